@@ -134,6 +134,22 @@ constexpr int kCsrLongRow = B2S_CSR_LONG_ROW;
 // nonzeros run the row-group CSR kernel.
 constexpr int kCsrGroupCap = 256;
 
+// Row patterns: the distinct sequences of column - row among a matrix's rows
+// (stencils have a few dozen), kept when there are at most kMaxPatterns of
+// them with kMaxPatternOffsets offsets in all and no row longer than
+// kMaxPatternRow. A product then reads one byte per row instead of four per
+// stored element for its columns.
+constexpr int kMaxPatterns = 255;
+constexpr int kMaxPatternOffsets = 2048;
+constexpr int kMaxPatternRow = 64;
+struct RowPatterns
+{
+   int32_t n, noff;       // patterns, their offsets in all
+   const int32_t* ptr;    // pattern p: offsets [ptr[p], ptr[p+1])
+   const int32_t* off;    // column - row
+   const uint8_t* id;     // pattern of each row (BiEllpack: of each strip rank)
+};
+
 struct ChunkSlice
 {
    int32_t size, chunkSize, firstSegment, pointer;
@@ -218,6 +234,10 @@ struct b2s_matrix_t
    // holds their count and alignedSize TNL's nonemptyRows
    b2s::DevBuf diagOffsets;
 
+   // row patterns (npat == 0: none): pointers, offsets, then a byte per row
+   b2s::DevBuf pat;
+   int32_t npat = 0, npat_off = 0;
+
    // Jacobi diagonal (matrix dtype)
    b2s::DevBuf diagonal;
    // staging buffers of the host-vector SpMV path (grown on demand; calls on
@@ -229,9 +249,23 @@ struct b2s_matrix_t
    std::unique_ptr< b2s::HostPipe > pipe;
 
    int64_t device_bytes() const;
+
+   b2s::RowPatterns patterns() const
+   {
+      const int32_t* p = pat.as< int32_t >();
+      return b2s::RowPatterns{ npat, npat_off, p, p + b2s::kMaxPatterns + 1,
+                               reinterpret_cast< const uint8_t* >( p + b2s::kMaxPatterns + 1 + b2s::kMaxPatternOffsets ) };
+   }
 };
 
 namespace b2s {
+
+// padded layouts: padding is more than a quarter of the stored elements
+inline bool
+much_padding( const b2s_matrix_t* A )
+{
+   return (double) A->alloc_elems > 1.25 * (double) ( A->nnz > 1 ? A->nnz : 1 );
+}
 
 // ---------------------------------------------------------------------------
 // Device helpers
@@ -338,6 +372,8 @@ constexpr int kMaxReduceGrid = 148 * 16;
 // Resident blocks per SM of `kernel` launched with `block` threads and no
 // dynamic shared memory (occupancy calculator, cached per kernel and device).
 int resident_blocks( const void* kernel, int block );
+// Lets `kernel` be launched with `bytes` of dynamic shared memory.
+b2s_status allow_smem( const void* kernel, size_t bytes );
 
 // Scratch owned by a handle: NR*kMaxReduceGrid doubles + counters.
 struct Scratch
@@ -374,6 +410,9 @@ b2s_status device_status( b2s_matrix_t* A, cudaStream_t s );
 // ---------------------------------------------------------------------------
 // Matrix helpers (matrix.cu)
 b2s_status build_diagonal( b2s_matrix_t* A, cudaStream_t s );
+// The row patterns of A as it is stored now (none when they do not fit the
+// limits or no kernel of A's would use them); again after its columns change.
+b2s_status build_row_patterns( b2s_matrix_t* A, cudaStream_t s );
 // The storage arrays of a padded layout as TNL keeps them (host side), e.g.
 // read from a file. Values are in `dtype`, `alloc` of them.
 // SymmetricMatrix (matrix.cu): check that a CSR matrix holds its lower

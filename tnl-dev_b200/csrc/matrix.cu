@@ -17,6 +17,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstddef>
 #include <cstring>
 #include <memory>
 
@@ -33,7 +34,7 @@ b2s_matrix_t::device_bytes() const
    const b2s::DevBuf* bufs[] = { &values,      &columns,           &values32,     &offsets,    &csr_win[ 0 ],
                                  &csr_win[ 1 ], &sliceOffsets, &sliceSegmentSizes, &rowToChunk,   &rowToSlice, &chunksToSeg,
                                  &rowPointers,  &cslices,           &rowPerm,      &groupPointers, &diagonal,
-                                 &rankRow,      &diagOffsets };
+                                 &rankRow,      &diagOffsets,       &pat };
    int64_t t = 0;
    for( auto* b : bufs )
       t += (int64_t) b->bytes;
@@ -232,6 +233,154 @@ layout_rows_kernel( LayoutView L, int32_t rows, int32_t segmentSize, const int32
       }
       if( ! WRITE )
          counts[ r ] = o;
+   }
+}
+
+// ---------------------------------------------------------------------------
+// Row patterns (RowPatterns): a hash of every row's offsets goes into a small
+// table with the first row that has it; the table's rows become the
+// dictionary; then every row is compared with its entry, element by element,
+// so equal hashes of different rows end in "no patterns" and not in a wrong
+// column.
+constexpr int kPatternTable = 1024;
+struct PatternWork
+{
+   unsigned long long key[ kPatternTable ];  // 0: free
+   int32_t row[ kPatternTable ];             // first row with this key
+   int32_t id[ kPatternTable ];
+   int32_t count;                            // keys in the table
+   int32_t failed;
+   int32_t noff;
+   int32_t pad;
+};
+
+// key of a row's offsets (never 0) and their number; -1: padding before an
+// element or too long a row
+__device__ __forceinline__ unsigned long long
+pattern_key( const LayoutView& L, int32_t segmentSize, const int32_t* __restrict__ col, int row, int& len )
+{
+   const int64_t cap = L.capacity( row, segmentSize );
+   unsigned long long h = 0x9E3779B97F4A7C15ull;
+   bool ended = false;
+   len = 0;
+   for( int64_t k = 0; k < cap; k++ ) {
+      const int64_t g = L.gidx( row, (int) k );
+      if( g < 0 )
+         break;
+      const int c = col[ g ];
+      if( c == -1 ) {
+         ended = true;
+         continue;
+      }
+      if( ended || len == kMaxPatternRow ) {
+         len = -1;
+         return 0;
+      }
+      h = ( h ^ (unsigned int) ( c - row ) ) * 0xD6E8FEB86659FD93ull;
+      h ^= h >> 32;
+      len++;
+   }
+   return h | 1ull;
+}
+
+__global__ void
+pattern_hash_kernel( LayoutView L, int32_t rows, int32_t segmentSize, const int32_t* __restrict__ col, PatternWork* W )
+{
+   for( int64_t r = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; r < rows; r += (int64_t) gridDim.x * blockDim.x ) {
+      if( *(volatile int32_t*) &W->failed )
+         return;
+      int len;
+      const unsigned long long key = pattern_key( L, segmentSize, col, (int) r, len );
+      if( len < 0 ) {
+         W->failed = 1;
+         return;
+      }
+      for( int probe = 0, t = (int) ( key >> 20 ) & ( kPatternTable - 1 ); probe < kPatternTable;
+           probe++, t = ( t + 1 ) & ( kPatternTable - 1 ) ) {
+         unsigned long long have = *(volatile unsigned long long*) &W->key[ t ];
+         if( have == 0 ) {
+            have = atomicCAS( &W->key[ t ], 0ull, key );
+            if( have == 0 ) {
+               have = key;
+               if( atomicAdd( &W->count, 1 ) >= kMaxPatterns )
+                  W->failed = 1;
+            }
+         }
+         if( have == key ) {
+            if( *(volatile int32_t*) &W->row[ t ] > (int) r )
+               atomicMin( &W->row[ t ], (int) r );
+            break;
+         }
+      }
+   }
+}
+
+// one block of kPatternTable threads: patterns numbered by their first row
+__global__ void __launch_bounds__( kPatternTable )
+pattern_dictionary_kernel( LayoutView L, int32_t segmentSize, const int32_t* __restrict__ col, PatternWork* W,
+                           int32_t* __restrict__ ptr, int32_t* __restrict__ out )
+{
+   __shared__ int32_t srow[ kPatternTable ], slen[ kMaxPatterns + 1 ];
+   const int t = threadIdx.x;
+   if( W->failed )
+      return;  // the same value for every thread: nothing writes it here before the barrier
+   const bool used = W->key[ t ] != 0;
+   const int row = used ? W->row[ t ] : INT32_MAX;
+   srow[ t ] = row;
+   __syncthreads();
+   int id = 0, len = 0;
+   if( used ) {
+      for( int q = 0; q < kPatternTable; q++ )
+         id += srow[ q ] < row;
+      pattern_key( L, segmentSize, col, row, len );
+      slen[ id ] = len;
+      W->id[ t ] = id;
+   }
+   __syncthreads();
+   const int n = W->count;
+   if( t == 0 ) {
+      int sum = 0;
+      for( int q = 0; q < n; q++ ) {
+         const int l = slen[ q ];
+         slen[ q ] = sum;
+         ptr[ q ] = sum;
+         sum += l;
+      }
+      ptr[ n ] = sum;
+      W->noff = sum;
+      if( sum > kMaxPatternOffsets )
+         W->failed = 1;
+      srow[ 0 ] = sum;
+   }
+   __syncthreads();
+   if( srow[ 0 ] > kMaxPatternOffsets || ! used )
+      return;
+   for( int k = 0; k < len; k++ )
+      out[ slen[ id ] + k ] = col[ L.gidx( row, k ) ] - row;
+}
+
+__global__ void
+pattern_assign_kernel( LayoutView L, int32_t rows, int32_t segmentSize, const int32_t* __restrict__ col, PatternWork* W,
+                       const int32_t* __restrict__ ptr, const int32_t* __restrict__ offs, uint8_t* __restrict__ id )
+{
+   if( W->failed )
+      return;
+   for( int64_t r = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; r < rows; r += (int64_t) gridDim.x * blockDim.x ) {
+      int len;
+      const unsigned long long key = pattern_key( L, segmentSize, col, (int) r, len );
+      int p = -1;
+      for( int probe = 0, t = (int) ( key >> 20 ) & ( kPatternTable - 1 ); probe < kPatternTable && p < 0;
+           probe++, t = ( t + 1 ) & ( kPatternTable - 1 ) )
+         if( W->key[ t ] == key )
+            p = W->id[ t ];
+      bool same = p >= 0 && ptr[ p + 1 ] - ptr[ p ] == len;
+      for( int k = 0; same && k < len; k++ )
+         same = col[ L.gidx( (int) r, k ) ] - (int) r == offs[ ptr[ p ] + k ];
+      if( ! same ) {
+         W->failed = 1;
+         return;
+      }
+      id[ L.format == B2S_BIELLPACK ? L.rowPerm[ r ] : r ] = (uint8_t) p;
    }
 }
 
@@ -814,6 +963,7 @@ build_from_device_csr( b2s_matrix_t* m, const int32_t* off, const int32_t* col, 
       // short, even rows: the row-group kernel
       m->csr_group_opt = opts.csr_row_groups;
       m->csr_group = hflags[ 2 ] <= kCsrGroupCap && opts.csr_row_groups >= 0 ? 1 : 0;
+      B2S_TRY( build_row_patterns( m, s ) );
       B2S_TRY_CUDA( cudaStreamSynchronize( s ) );
       return B2S_OK;
    }
@@ -938,6 +1088,7 @@ build_from_device_csr( b2s_matrix_t* m, const int32_t* off, const int32_t* col, 
    }
    // count the nonzeros that survived (zeros dropped)
    m->nnz = nnz;
+   B2S_TRY( build_row_patterns( m, s ) );
    B2S_TRY_CUDA( cudaStreamSynchronize( s ) );
    return B2S_OK;
 }
@@ -1250,16 +1401,18 @@ clone_matrix( const b2s_matrix_t* a, b2s_matrix_t* m, cudaStream_t s )
    m->slice_size = a->slice_size;
    m->numberOfSlices = a->numberOfSlices;
    m->virtualRows = a->virtualRows;
+   m->npat = a->npat;
+   m->npat_off = a->npat_off;
    const b2s::DevBuf* from[] = { &a->values,        &a->columns,      &a->values32,    &a->offsets,
                                  &a->csr_win[ 0 ],  &a->csr_win[ 1 ], &a->sliceOffsets, &a->sliceSegmentSizes,
                                  &a->rowToChunk,    &a->rowToSlice,   &a->chunksToSeg, &a->rowPointers,
                                  &a->cslices,       &a->rowPerm,      &a->groupPointers, &a->diagonal,
-                                 &a->rankRow };
+                                 &a->rankRow,       &a->pat };
    b2s::DevBuf* to[] = { &m->values,        &m->columns,      &m->values32,    &m->offsets,
                          &m->csr_win[ 0 ],  &m->csr_win[ 1 ], &m->sliceOffsets, &m->sliceSegmentSizes,
                          &m->rowToChunk,    &m->rowToSlice,   &m->chunksToSeg, &m->rowPointers,
                          &m->cslices,       &m->rowPerm,      &m->groupPointers, &m->diagonal,
-                         &m->rankRow };
+                         &m->rankRow,       &m->pat };
    for( size_t i = 0; i < sizeof( from ) / sizeof( from[ 0 ] ); i++ )
       B2S_TRY( dup_buf( *to[ i ], *from[ i ], s ) );
    B2S_TRY( m->status.alloc( 4 * sizeof( int ) ) );
@@ -1428,6 +1581,7 @@ matrix_from_layout( const LayoutArrays& L, const b2s_matrix_opts& o, cudaStream_
    B2S_TRY( build_diagonal( m.get(), s ) );
    if( o.keep_fp32_copy )
       B2S_TRY( ensure_fp32_copy( m.get(), s ) );
+   B2S_TRY( build_row_patterns( m.get(), s ) );
    B2S_TRY_CUDA( cudaStreamSynchronize( s ) );
    *out = m.release();
    return B2S_OK;
@@ -1626,6 +1780,51 @@ expand_symmetric( const b2s_matrix_t* src, cudaStream_t s, b2s_matrix_t** out )
                                  tj.as< int32_t >(), tv.p, (b2s_dtype) m->dtype, B2S_DEVICE, B2S_DUP_ADD, nullptr, &o,
                                  s, &g ) );
    *out = g;
+   return B2S_OK;
+}
+
+b2s_status
+build_row_patterns( b2s_matrix_t* A, cudaStream_t s )
+{
+   A->npat = 0;
+   A->npat_off = 0;
+   A->pat.release();
+   // the kernels that read patterns: CSR row groups and the padded layouts
+   // where padding is rare
+   const bool csr = A->format == B2S_CSR && A->csr_kernel == B2S_CSR_ADAPTIVE && A->csr_group;
+   const bool padded = A->format == B2S_ELLPACK || A->format == B2S_SLICED_ELLPACK || A->format == B2S_BIELLPACK
+                       || ( A->format == B2S_CHUNKED_ELLPACK && A->chunk_single );
+   if( ! ( csr || ( padded && ! much_padding( A ) ) ) || A->symmetric || A->dtype == B2S_BOOL || A->rows == 0
+       || A->nnz == 0 || ( csr && A->max_row > kMaxPatternRow ) )
+      return B2S_OK;
+   const int32_t rows = A->rows;
+   const int64_t ids = A->format == B2S_BIELLPACK ? A->virtualRows : rows;
+   DevBuf work;
+   B2S_TRY( work.alloc( sizeof( PatternWork ) ) );
+   B2S_TRY_CUDA( cudaMemsetAsync( work.p, 0, sizeof( PatternWork ), s ) );
+   B2S_TRY_CUDA( cudaMemsetAsync( reinterpret_cast< char* >( work.p ) + offsetof( PatternWork, row ), 0x7f,
+                                  sizeof( PatternWork::row ), s ) );
+   B2S_TRY( A->pat.alloc( ( kMaxPatterns + 1 + kMaxPatternOffsets ) * sizeof( int32_t ) + (size_t) ids ) );
+   // ids of strip ranks past the rows: pattern 0, never stored
+   B2S_TRY_CUDA( cudaMemsetAsync( A->pat.p, 0, A->pat.bytes, s ) );
+   int32_t* ptr = A->pat.as< int32_t >();
+   int32_t* off = ptr + kMaxPatterns + 1;
+   uint8_t* id = reinterpret_cast< uint8_t* >( off + kMaxPatternOffsets );
+   PatternWork* W = work.as< PatternWork >();
+   const LayoutView L = view_of( A );
+   const int32_t* col = A->columns.as< int32_t >();
+   pattern_hash_kernel<<< grid_for( rows ), 256, 0, s >>>( L, rows, A->segmentSize, col, W );
+   pattern_dictionary_kernel<<< 1, kPatternTable, 0, s >>>( L, A->segmentSize, col, W, ptr, off );
+   pattern_assign_kernel<<< grid_for( rows ), 256, 0, s >>>( L, rows, A->segmentSize, col, W, ptr, off, id );
+   B2S_TRY_CUDA( cudaGetLastError() );
+   int32_t h[ 3 ];  // count, failed, noff
+   B2S_TRY( copy_d2h( h, reinterpret_cast< char* >( work.p ) + offsetof( PatternWork, count ), sizeof( h ), s ) );
+   if( h[ 1 ] || h[ 0 ] == 0 ) {
+      A->pat.release();
+      return B2S_OK;
+   }
+   A->npat = h[ 0 ];
+   A->npat_off = h[ 2 ];
    return B2S_OK;
 }
 

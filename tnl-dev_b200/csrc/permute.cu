@@ -234,6 +234,7 @@ b2s_matrix_permute_columns( b2s_matrix A, const int32_t* iperm, b2s_memory where
    }
    // the Jacobi diagonal follows the new column indices
    B2S_TRY( build_diagonal( A, s ) );
+   B2S_TRY( build_row_patterns( A, s ) );
    B2S_TRY_CUDA( cudaStreamSynchronize( s ) );
    return B2S_OK;
 }

@@ -73,6 +73,23 @@ resident_blocks( const void* kernel, int block )
    return occ;
 }
 
+b2s_status
+allow_smem( const void* kernel, size_t bytes )
+{
+   if( bytes <= 48 * 1024 )
+      return B2S_OK;
+   static std::mutex mu;
+   static std::map< std::pair< const void*, int >, size_t > allowed;
+   const auto key = std::make_pair( kernel, current_device() );
+   std::lock_guard< std::mutex > lock( mu );
+   size_t& a = allowed[ key ];
+   if( bytes > a ) {
+      B2S_TRY_CUDA( cudaFuncSetAttribute( kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes ) );
+      a = bytes;
+   }
+   return B2S_OK;
+}
+
 int
 reduce_grid( int64_t n, int per_thread )
 {

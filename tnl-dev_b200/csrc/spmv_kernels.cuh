@@ -557,6 +557,380 @@ csr_group_kernel( const int32_t* __restrict__ off, const int32_t* __restrict__ c
 }
 
 // ---------------------------------------------------------------------------
+// Row patterns (RowPatterns): the columns of a row are row + a short list of
+// offsets that a few dozen patterns share, so a product reads the row's
+// pattern number (one byte) instead of its columns (four bytes per element),
+// and the gathers of x no longer wait for a column load. The lists sit in
+// shared memory; a warp's rows nearly always have one pattern, whose offsets
+// are then broadcast.
+struct PatternSmem
+{
+   int32_t ptr[ kMaxPatterns + 1 ];
+   int32_t off[ kMaxPatternOffsets ];
+};
+
+// the caller synchronizes the block before the lists are used
+template< int BLOCK >
+__device__ __forceinline__ void
+load_patterns( const RowPatterns& P, PatternSmem& S )
+{
+   for( int i = threadIdx.x; i <= P.n; i += BLOCK )
+      S.ptr[ i ] = __ldg( P.ptr + i );
+   for( int i = threadIdx.x; i < P.noff; i += BLOCK )
+      S.off[ i ] = __ldg( P.off + i );
+}
+
+// CSR row groups with patterns: csr_group_kernel without the columns. The
+// row-group kernels issue instructions most of the time (0.6-0.7 per cycle and
+// scheduler), so this one counts them: 32-bit row arithmetic, eight elements at
+// a time under predicates.
+// Groups of values in flight or being summed per warp: three in FP32, whose
+// groups carry half the bytes (128^3 / 160^3 Laplacian 24.7 / 41.4 us against
+// 28.5 / 49.6 us with two), two in FP64 (33.1 against 34.3 us with three).
+template< typename Real >
+constexpr int kCsrPatStages = sizeof( Real ) == 4 ? 3 : 2;
+template< typename Real, class Sink >
+__global__ void __launch_bounds__( kCsrGroupBlock, 8 )
+csr_pattern_kernel( const int32_t* __restrict__ off, RowPatterns P, const Real* __restrict__ val,
+                    const Real* __restrict__ x, int32_t row_begin, int32_t row_end, Sink sink, RedScratch rs )
+{
+   constexpr int VPC = 16 / sizeof( Real );  // values per 16-byte chunk
+   constexpr int SC = kCsrGroupCap + 8;      // room for the alignment slack
+   constexpr int NS = kCsrPatStages< Real >;
+   __shared__ __align__( 16 ) Real sval[ kCsrGroupWarps ][ NS ][ SC ];
+   __shared__ PatternSmem sp;
+   if( sink.skip() )
+      return;  // uniform over the grid: the solve this launch belongs to is finished
+   AccOf< Sink > acc{};
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+   const uint64_t pol = l2_evict_first();
+   // this warp's groups start at rows row, row + step, ... (below 2^31 + step: kept unsigned)
+   const unsigned end = (unsigned) row_end;
+   const unsigned step = gridDim.x * kCsrGroupWarps * kCsrGroupRows;
+   unsigned row = (unsigned) row_begin + ( blockIdx.x * kCsrGroupWarps + warp ) * kCsrGroupRows;
+   // this lane's row start and pattern in the group from g0 (dead lanes: the end of the last row)
+   auto load_row = [ & ]( unsigned g0, int& lo, int& p )
+   {
+      const unsigned r = min( g0 + lane, end );
+      lo = 0;
+      p = -1;
+      if( g0 < end ) {
+         lo = __ldg( off + r );
+         if( r < end )
+            p = __ldg( P.id + r );
+      }
+   };
+   // the group's values: from lane 0's row start to the end of lane 31's row
+   auto stage = [ & ]( unsigned g0, int lo, int p, int buf )
+   {
+      if( g0 < end ) {
+         const int len = p >= 0 ? sp.ptr[ p + 1 ] - sp.ptr[ p ] : 0;
+         const int v0 = __shfl_sync( 0xffffffffu, lo, 0 ) & ~( VPC - 1 );
+         const int n = __shfl_sync( 0xffffffffu, lo + len, 31 ) - v0;
+         const Real* src = val + v0;
+         Real* dst = sval[ warp ][ buf ];
+         for( int q = VPC * lane; q < n; q += 32 * VPC )
+            cp_async16( dst + q, src + q, pol );
+      }
+      cp_async_commit();  // an empty group past the end keeps the wait counts uniform
+   };
+   int lo[ NS ], pn[ NS ];
+#pragma unroll
+   for( int i = 0; i < NS; i++ )
+      load_row( row + i * step, lo[ i ], pn[ i ] );
+   load_patterns< kCsrGroupBlock >( P, sp );
+   __syncthreads();
+#pragma unroll
+   for( int i = 0; i < NS - 1; i++ )
+      stage( row + i * step, lo[ i ], pn[ i ], i );
+   int buf = 0;
+   for( ; row < end; row += step ) {
+      stage( row + ( NS - 1 ) * step, lo[ NS - 1 ], pn[ NS - 1 ], buf == 0 ? NS - 1 : buf - 1 );
+      int nlo, np;
+      load_row( row + NS * step, nlo, np );
+      const int first = lo[ 0 ], p = pn[ 0 ];
+      const int pb = p >= 0 ? sp.ptr[ p ] : 0, len = p >= 0 ? sp.ptr[ p + 1 ] - pb : 0;
+      const int* so = sp.off + pb;
+      const Real* xr = x + ( row + lane );
+      // the gathers of the row's first elements need no column and go out
+      // before the wait for the values
+      Real xv[ 8 ];
+#pragma unroll
+      for( int i = 0; i < 8; i++ )
+         xv[ i ] = i < len ? __ldg( xr + so[ i ] ) : Real( 0 );
+      const Real* sv = sval[ warp ][ buf ] + ( first - ( __shfl_sync( 0xffffffffu, first, 0 ) & ~( VPC - 1 ) ) );
+      cp_async_wait< NS - 1 >();  // this group's copies have landed
+      __syncwarp();
+      Real sum = 0;
+#pragma unroll
+      for( int i = 0; i < 8; i++ )
+         if( i < len )
+            sum = sum + mul_rn( sv[ i ], xv[ i ] );
+      for( int k = 8; k < len; k += 8 ) {
+#pragma unroll
+         for( int i = 0; i < 8; i++ )
+            xv[ i ] = k + i < len ? __ldg( xr + so[ k + i ] ) : Real( 0 );
+#pragma unroll
+         for( int i = 0; i < 8; i++ )
+            if( k + i < len )
+               sum = sum + mul_rn( sv[ k + i ], xv[ i ] );
+      }
+      if( p >= 0 )
+         sink.put( (int) ( row + lane ), sum, acc.v );
+      __syncwarp();  // the buffer is refilled NS groups later
+#pragma unroll
+      for( int i = 0; i < NS - 1; i++ ) {
+         lo[ i ] = lo[ i + 1 ];
+         pn[ i ] = pn[ i + 1 ];
+      }
+      lo[ NS - 1 ] = nlo;
+      pn[ NS - 1 ] = np;
+      buf = buf + 1 == NS ? 0 : buf + 1;
+   }
+   cp_async_wait< 0 >();
+   spmv_epilogue< Sink, kCsrGroupBlock >( sink, acc.v, rs );
+}
+
+// R adjacent values, one load (val + g aligned to their size)
+__device__ __forceinline__ void
+ld_values( const float* p, float ( &v )[ 4 ] )
+{
+   const float4 q = __ldcs( reinterpret_cast< const float4* >( p ) );
+   v[ 0 ] = q.x;
+   v[ 1 ] = q.y;
+   v[ 2 ] = q.z;
+   v[ 3 ] = q.w;
+}
+__device__ __forceinline__ void
+ld_values( const float* p, float ( &v )[ 2 ] )
+{
+   const float2 q = __ldcs( reinterpret_cast< const float2* >( p ) );
+   v[ 0 ] = q.x;
+   v[ 1 ] = q.y;
+}
+__device__ __forceinline__ void
+ld_values( const double* p, double ( &v )[ 2 ] )
+{
+   const double2 q = __ldcs( reinterpret_cast< const double2* >( p ) );
+   v[ 0 ] = q.x;
+   v[ 1 ] = q.y;
+}
+__device__ __forceinline__ void
+ld_values( const double* p, double ( &v )[ 4 ] )
+{
+   asm( "ld.global.nc.L1::no_allocate.v4.f64 {%0,%1,%2,%3}, [%4];"
+        : "=d"( v[ 0 ] ), "=d"( v[ 1 ] ), "=d"( v[ 2 ] ), "=d"( v[ 3 ] )
+        : "l"( p ) );
+}
+
+// slots whose loads are in flight together, per row of a thread (eight took
+// the registers of three resident blocks: 37 against 31 us on the 128^3
+// Laplacian in FP64)
+constexpr int kPatternUnroll = 4;
+
+// Ellpack and SlicedEllpack with patterns, R adjacent rows per thread (r a
+// multiple of R, slots of neighbouring rows neighbours): the values of slot k
+// are one load, no columns are read. SLICED: slice size 1 << shift; otherwise
+// the slots of row r are r + stride * k. Each row's sum runs over its slots in
+// order, as in the kernels that read columns.
+template< typename Real, int R, bool SLICED, class Sink >
+__global__ void __launch_bounds__( kSpmvBlock )
+ellpack_pattern_kernel( RowPatterns P, const Real* __restrict__ val, const int32_t* __restrict__ sliceOffsets,
+                        int32_t shift, int32_t stride, const Real* __restrict__ x, int32_t row_begin, int32_t row_end,
+                        Sink sink, RedScratch rs )
+{
+   __shared__ PatternSmem sp;
+   if( sink.skip() )
+      return;
+   AccOf< Sink > acc{};
+   load_patterns< kSpmvBlock >( P, sp );
+   __syncthreads();
+   // rows below 2^31 + a step of the grid: kept unsigned; the next step's
+   // pattern numbers and slice starts are loaded one step ahead
+   const unsigned end = (unsigned) row_end, hop = R * gridDim.x * kSpmvBlock;
+   unsigned r = (unsigned) row_begin + R * ( blockIdx.x * kSpmvBlock + threadIdx.x );
+   int p[ R ], base = 0;
+   auto fetch = [ & ]( unsigned q )
+   {
+#pragma unroll
+      for( int j = 0; j < R; j++ )
+         p[ j ] = q + j < end ? __ldg( P.id + q + j ) : -1;
+      if( SLICED && q < end )
+         base = __ldg( sliceOffsets + ( q >> shift ) );
+   };
+   fetch( r );
+   for( ; r < end; r += hop ) {
+      const Real* v0 = val + ( SLICED ? base + (int) ( r & ( ( 1u << shift ) - 1 ) ) : (int) r );
+      const int *so[ R ];
+      int len[ R ], most = 0;
+      bool live[ R ];
+      Real s[ R ];
+#pragma unroll
+      for( int j = 0; j < R; j++ ) {
+         live[ j ] = p[ j ] >= 0;
+         const int pb = live[ j ] ? sp.ptr[ p[ j ] ] : 0;
+         len[ j ] = live[ j ] ? sp.ptr[ p[ j ] + 1 ] - pb : 0;
+         so[ j ] = sp.off + pb;
+         most = max( most, len[ j ] );
+         s[ j ] = 0;
+      }
+      fetch( r + hop );
+      const Real* xr = x + r;
+      for( int k = 0; k < most; k += kPatternUnroll ) {
+         Real v[ kPatternUnroll ][ R ], xv[ kPatternUnroll ][ R ];
+#pragma unroll
+         for( int i = 0; i < kPatternUnroll; i++ )
+            if( k + i < most ) {
+               ld_values( v0 + (int64_t) ( k + i ) * stride, v[ i ] );
+#pragma unroll
+               for( int j = 0; j < R; j++ )
+                  xv[ i ][ j ] = k + i < len[ j ] ? __ldg( xr + j + so[ j ][ k + i ] ) : Real( 0 );
+            }
+#pragma unroll
+         for( int i = 0; i < kPatternUnroll; i++ )
+#pragma unroll
+            for( int j = 0; j < R; j++ )
+               if( k + i < len[ j ] )
+                  s[ j ] += v[ i ][ j ] * xv[ i ][ j ];
+      }
+#pragma unroll
+      for( int j = 0; j < R; j++ )
+         if( live[ j ] )
+            sink.put( (int) r + j, s[ j ], acc.v );
+   }
+   spmv_epilogue< Sink, kSpmvBlock >( sink, acc.v, rs );
+}
+
+// ChunkedEllpack with one chunk per row (chunked1_kernel) with patterns.
+template< typename Real, class Sink >
+__global__ void __launch_bounds__( kChunksInSlice )
+chunked_pattern_kernel( RowPatterns P, const Real* __restrict__ val, const ChunkSlice* __restrict__ slices,
+                        const int32_t* __restrict__ rowToSlice, const Real* __restrict__ x, int32_t row_begin,
+                        int32_t row_end, Sink sink, RedScratch rs )
+{
+   __shared__ PatternSmem sp;
+   if( sink.skip() )
+      return;
+   AccOf< Sink > acc{};
+   load_patterns< kChunksInSlice >( P, sp );
+   __syncthreads();
+   const int s_first = __ldg( rowToSlice + row_begin );
+   const int s_last = __ldg( rowToSlice + row_end - 1 );
+   for( int sidx = s_first + blockIdx.x; sidx <= s_last; sidx += gridDim.x ) {
+      const ChunkSlice sl = slices[ sidx ];
+      const int row = sl.firstSegment + (int) threadIdx.x;
+      if( (int) threadIdx.x < sl.size && row >= row_begin && row < row_end ) {
+         const int p = __ldg( P.id + row );
+         const int pb = sp.ptr[ p ], len = sp.ptr[ p + 1 ] - pb;
+         const Real* vr = val + sl.pointer + threadIdx.x;
+         const Real* xr = x + row;
+         Real s = 0;
+#pragma unroll 8
+         for( int k = 0; k < len; k++ )
+            s += ld_stream( vr + (int64_t) k * kChunksInSlice ) * __ldg( xr + sp.off[ pb + k ] );
+         Real t = 0;
+         t += s;
+         sink.put( row, t, acc.v );
+      }
+   }
+   spmv_epilogue< Sink, kChunksInSlice >( sink, acc.v, rs );
+}
+
+// BiEllpack by rank pairs (biell_pair_kernel) with patterns, whose numbers are
+// stored in rank order.
+template< typename Real, class Sink >
+__global__ void __launch_bounds__( kSpmvBlock )
+biell_pattern_kernel( RowPatterns P, const Real* __restrict__ val, const int32_t* __restrict__ rankRow,
+                      const int32_t* __restrict__ groupPointers, const Real* __restrict__ x, int32_t row_begin,
+                      int32_t row_end, Sink sink, RedScratch rs )
+{
+   __shared__ PatternSmem sp;
+   if( sink.skip() )
+      return;
+   AccOf< Sink > acc{};
+   load_patterns< kSpmvBlock >( P, sp );
+   __syncthreads();
+   const int lane = threadIdx.x & 31, half = lane >> 4, q = lane & 15;
+   const int64_t warp_global = ( blockIdx.x * (int64_t) kSpmvBlock + threadIdx.x ) >> 5;
+   const int64_t nwarps = ( (int64_t) gridDim.x * kSpmvBlock ) >> 5;
+   const int64_t first = row_begin / kBiWarp, last = ( (int64_t) row_end - 1 ) / kBiWarp;
+   for( int64_t pair = warp_global; first + 2 * pair <= last; pair += nwarps ) {
+      const int64_t strip = first + 2 * pair + half;
+      const bool live = strip <= last;
+      int gpl = 0;
+      if( live && q <= kBiGroups )
+         gpl = __ldg( groupPointers + strip * kBiGroups + q );
+      int row[ 2 ] = { -1, -1 }, pb[ 2 ] = { 0, 0 }, len[ 2 ] = { 0, 0 };
+      if( live ) {
+         const int2 rr = __ldg( reinterpret_cast< const int2* >( rankRow + strip * kBiWarp + 2 * q ) );
+         row[ 0 ] = rr.x;
+         row[ 1 ] = rr.y;
+#pragma unroll
+         for( int j = 0; j < 2; j++ ) {
+            const int p = __ldg( P.id + strip * kBiWarp + 2 * q + j );
+            if( row[ j ] >= row_begin && row[ j ] < row_end ) {
+               pb[ j ] = sp.ptr[ p ];
+               len[ j ] = sp.ptr[ p + 1 ] - pb[ j ];
+            }
+            else
+               row[ j ] = -1;
+         }
+      }
+      int gpk[ kBiGroups + 1 ];
+#pragma unroll
+      for( int k = 0; k <= kBiGroups; k++ )
+         gpk[ k ] = __shfl_sync( 0xffffffffu, gpl, ( lane & 16 ) + k );
+      Real s[ 2 ] = { 0, 0 };
+      // group 0: all 32 ranks, 32 slots per element position
+      const int w0 = ( gpk[ 1 ] - gpk[ 0 ] ) >> 5;
+      const int m0 = min( w0, max( len[ 0 ], len[ 1 ] ) );
+      const Real* v0 = val + (int64_t) gpk[ 0 ] + 2 * q;
+      const Real* x0 = x + row[ 0 ];
+      const Real* x1 = x + row[ 1 ];
+      if( ( gpk[ 0 ] & 1 ) == 0 ) {
+#pragma unroll 4
+         for( int k = 0; k < m0; k++ ) {
+            Real v[ 2 ];
+            ld_values( v0 + k * kBiWarp, v );
+            if( k < len[ 0 ] )
+               s[ 0 ] += v[ 0 ] * __ldg( x0 + sp.off[ pb[ 0 ] + k ] );
+            if( k < len[ 1 ] )
+               s[ 1 ] += v[ 1 ] * __ldg( x1 + sp.off[ pb[ 1 ] + k ] );
+         }
+      }
+      else {
+#pragma unroll 4
+         for( int k = 0; k < m0; k++ ) {
+            if( k < len[ 0 ] )
+               s[ 0 ] += ld_stream( v0 + k * kBiWarp ) * __ldg( x0 + sp.off[ pb[ 0 ] + k ] );
+            if( k < len[ 1 ] )
+               s[ 1 ] += ld_stream( v0 + k * kBiWarp + 1 ) * __ldg( x1 + sp.off[ pb[ 1 ] + k ] );
+         }
+      }
+      // the higher groups, where a row goes on past group 0
+#pragma unroll
+      for( int j = 0; j < 2; j++ ) {
+         if( len[ j ] <= w0 )
+            continue;
+         int k = w0;
+         const Real* xj = x + row[ j ];
+#pragma unroll
+         for( int h = 1; h < kBiGroups; h++ ) {
+            const int w = ( gpk[ h + 1 ] - gpk[ h ] ) >> ( 5 - h );  // group h: 32 >> h ranks wide
+            const Real* vh = val + (int64_t) gpk[ h ] + 2 * q + j;
+            for( int i = 0; i < w && k < len[ j ]; i++, k++ )
+               s[ j ] += ld_stream( vh + i * ( kBiWarp >> h ) ) * __ldg( xj + sp.off[ pb[ j ] + k ] );
+         }
+      }
+#pragma unroll
+      for( int j = 0; j < 2; j++ )
+         if( row[ j ] >= 0 )
+            sink.put( row[ j ], s[ j ], acc.v );
+   }
+   spmv_epilogue< Sink, kSpmvBlock >( sink, acc.v, rs );
+}
+
+// ---------------------------------------------------------------------------
 // One slot of a padded layout into s. With SKIP the value of a padding slot
 // (column -1, value 0) is never read: where padding dominates (irregular rows
 // in Ellpack-like layouts) that removes most of the value bytes. Without it
@@ -1169,32 +1543,36 @@ constexpr int csr_group_rows_per_lane()
    return sizeof( Real ) == 4 ? B2S_CSR_GROUP_RPL_F32 : 1;
 }
 
-// the row-group kernel on the rows [rb, re) (rb a multiple of 32 RPL), over
-// the resident blocks only
+// grid of the row-group kernels on the rows [rb, re): the resident blocks only
+template< class Kernel >
+inline int
+csr_group_grid( Kernel kern, int32_t rb, int32_t re, int group_rows )
+{
+   const int occ = resident_blocks( reinterpret_cast< const void* >( kern ), kCsrGroupBlock );
+   const int64_t groups = ( (int64_t) re - rb + group_rows - 1 ) / group_rows;
+   const int64_t want = ( groups + kCsrGroupWarps - 1 ) / kCsrGroupWarps;
+   return (int) std::max< int64_t >( 1,
+                                     std::min< int64_t >( want, std::min< int64_t >( (int64_t) num_sms() * occ, kMaxReduceGrid ) ) );
+}
+
+// the row-group kernel on the rows [rb, re) (rb a multiple of 32 RPL)
 template< typename Real, int RPL, class Sink >
 inline b2s_status
 launch_csr_group( const int32_t* off, const int32_t* col, const Real* values, const Real* x, int32_t rb, int32_t re,
                   const Sink& sink, RedScratch rs, cudaStream_t s )
 {
    auto kern = csr_group_kernel< Real, RPL, Sink >;
-   static int per_sm[ 64 ] = {};
-   const int dev = current_device();
-   int occ = dev >= 0 && dev < 64 ? per_sm[ dev ] : 0;
-   if( occ == 0 ) {
-      B2S_TRY_CUDA( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, kern, kCsrGroupBlock, 0 ) );
-      occ = std::max( occ, 1 );
-      if( dev >= 0 && dev < 64 )
-         per_sm[ dev ] = occ;
-   }
-   const int64_t nr = (int64_t) re - rb;
-   const int64_t groups = ( nr + kCsrGroupRows * RPL - 1 ) / ( kCsrGroupRows * RPL );
-   const int64_t want = ( groups + kCsrGroupWarps - 1 ) / kCsrGroupWarps;
-   const int grid = (int) std::max< int64_t >(
-      1, std::min< int64_t >( want, std::min< int64_t >( (int64_t) num_sms() * occ, kMaxReduceGrid ) ) );
-   kern<<< grid, kCsrGroupBlock, 0, s >>>( off, col, values, x, rb, re, sink, rs );
+   kern<<< csr_group_grid( kern, rb, re, kCsrGroupRows * RPL ), kCsrGroupBlock, 0, s >>>( off, col, values, x, rb, re, sink,
+                                                                                         rs );
    B2S_TRY_CUDA( cudaGetLastError() );
    return B2S_OK;
 }
+
+// Rows per thread of the Ellpack-like pattern kernels: 16 bytes of values
+// (FP64: four rows were slower, 39 against 31 us on the 128^3 Laplacian; FP32:
+// two rows equal at 128^3, 37 against 35 us at 160^3)
+template< typename Real >
+constexpr int kPatternRows = 16 / sizeof( Real );
 
 template< typename Real, class Sink >
 inline b2s_status
@@ -1207,16 +1585,28 @@ spmv_dispatch( const b2s_matrix_t* A, const Real* values, const Real* x, int32_t
       return B2S_OK;
    // padded layouts: skip the value loads of padding slots when padding is
    // more than a quarter of the slots
-   const bool skip = (double) A->alloc_elems > 1.25 * (double) std::max< int64_t >( A->nnz, 1 );
+   const bool skip = much_padding( A );
    // the row-quad and row-pair kernels load 4 (2) neighbouring slots at once:
    // their base pointers must be aligned to those loads
    const bool quad_aligned = reinterpret_cast< uintptr_t >( values ) % ( 4 * sizeof( Real ) ) == 0
                              && reinterpret_cast< uintptr_t >( col ) % 16 == 0;
    const bool pair_aligned = reinterpret_cast< uintptr_t >( values ) % ( 2 * sizeof( Real ) ) == 0
                              && reinterpret_cast< uintptr_t >( col ) % 8 == 0;
+   // Row patterns: the columns are not read (see RowPatterns). The Ellpack-like
+   // kernels load R neighbouring slots at once, as the kernels below do.
+   constexpr int PR = kPatternRows< Real >;
+   const bool patterns = A->npat > 0;
+   const bool pat_rows =
+      patterns && reinterpret_cast< uintptr_t >( values ) % ( PR * sizeof( Real ) ) == 0 && rb % PR == 0;
    switch( A->format ) {
       case B2S_CSR: {
          const int32_t* off = A->offsets.as< int32_t >();
+         if( patterns && rb % kCsrGroupRows == 0 ) {
+            auto kern = csr_pattern_kernel< Real, Sink >;
+            kern<<< csr_group_grid( kern, rb, re, kCsrGroupRows ), kCsrGroupBlock, 0, s >>>( off, A->patterns(), values, x, rb,
+                                                                                           re, sink, rs );
+            break;
+         }
          if( A->csr_kernel == B2S_CSR_ADAPTIVE && A->csr_group && rb % kCsrGroupRows == 0 ) {
             constexpr int R2 = csr_group_rows_per_lane< Real >();
             if( R2 > 1 && rb % ( kCsrGroupRows * R2 ) == 0 )
@@ -1266,6 +1656,12 @@ spmv_dispatch( const b2s_matrix_t* A, const Real* values, const Real* x, int32_t
          break;
       }
       case B2S_ELLPACK:
+         if( pat_rows && A->alignedSize % PR == 0 ) {
+            ellpack_pattern_kernel< Real, PR, false, Sink ><<< spmv_grid( ( nr + PR - 1 ) / PR, kSpmvBlock ), kSpmvBlock, 0,
+                                                               s >>>( A->patterns(), values, nullptr, 0, A->alignedSize, x,
+                                                                      rb, re, sink, rs );
+            break;
+         }
          // row pairs where padding is rare (with much padding the pair's
          // shorter row would load values of its padding slots)
          if constexpr( kQuadRowsEllpack< Real > ) {
@@ -1286,6 +1682,15 @@ spmv_dispatch( const b2s_matrix_t* A, const Real* values, const Real* x, int32_t
                col, values, A->segmentSize, A->alignedSize, x, rb, re, sink, rs );
          break;
       case B2S_SLICED_ELLPACK: {
+         if( pat_rows ) {
+            int shift = 3;  // slices of 8, 16, 32 or 64 rows
+            while( ( 1 << shift ) < A->slice_size )
+               shift++;
+            ellpack_pattern_kernel< Real, PR, true, Sink ><<< spmv_grid( ( nr + PR - 1 ) / PR, kSpmvBlock ), kSpmvBlock, 0,
+                                                              s >>>( A->patterns(), values, A->sliceOffsets.as< int32_t >(),
+                                                                     shift, A->slice_size, x, rb, re, sink, rs );
+            break;
+         }
          const bool quad = kQuadRowsSliced< Real > && ! skip && quad_aligned && rb % 4 == 0;
          const bool pair = ! quad && ! skip && pair_aligned && rb % 2 == 0;
          const int grid = spmv_grid( quad ? ( nr + 3 ) / 4 : ( pair ? ( nr + 1 ) / 2 : nr ), kSpmvBlock );
@@ -1323,7 +1728,11 @@ spmv_dispatch( const b2s_matrix_t* A, const Real* values, const Real* x, int32_t
       case B2S_CHUNKED_ELLPACK: {
          const int grid = (int) std::min< int64_t >( std::max( A->numberOfSlices, 1 ),
                                                      std::min< int64_t >( (int64_t) num_sms() * 8, kMaxReduceGrid ) );
-         if( A->chunk_single ) {
+         if( patterns ) {
+            chunked_pattern_kernel< Real, Sink ><<< grid, kChunksInSlice, 0, s >>>(
+               A->patterns(), values, A->cslices.as< ChunkSlice >(), A->rowToSlice.as< int32_t >(), x, rb, re, sink, rs );
+         }
+         else if( A->chunk_single ) {
             if( skip )
                chunked1_kernel< Real, true, Sink ><<< grid, kChunksInSlice, 0, s >>>(
                   col, values, A->cslices.as< ChunkSlice >(), A->rowToSlice.as< int32_t >(), x, rb, re, sink, rs );
@@ -1342,7 +1751,12 @@ spmv_dispatch( const b2s_matrix_t* A, const Real* values, const Real* x, int32_t
          break;
       }
       case B2S_BIELLPACK:
-         if( A->rankRow.p && ! skip && pair_aligned ) {
+         if( patterns && A->rankRow.p && pair_aligned ) {
+            const int64_t lanes = ( ( (int64_t) re - 1 ) / kBiWarp - rb / kBiWarp + 2 ) / 2 * kBiWarp;
+            biell_pattern_kernel< Real, Sink ><<< spmv_grid( lanes, kSpmvBlock ), kSpmvBlock, 0, s >>>(
+               A->patterns(), values, A->rankRow.as< int32_t >(), A->groupPointers.as< int32_t >(), x, rb, re, sink, rs );
+         }
+         else if( A->rankRow.p && ! skip && pair_aligned ) {
             // rank pairs where padding is rare (a pair loads both ranks' values)
             const int64_t lanes = ( ( (int64_t) re - 1 ) / kBiWarp - rb / kBiWarp + 2 ) / 2 * kBiWarp;
             biell_pair_kernel< Real, false, Sink ><<< spmv_grid( lanes, kSpmvBlock ), kSpmvBlock, 0, s >>>(
