@@ -274,6 +274,159 @@ i64_to_i32_kernel( const int64_t* __restrict__ in, int64_t n, int32_t* __restric
       out[ i ] = (int32_t) in[ i ];
 }
 
+// ---------------------------------------------------------------------------
+// Assembly by rows. Sorting all triplets on row and column takes a pass of the
+// radix sort per eight bits of both (six for a 3000 x 3000 grid), each of
+// which moves every triplet; but only the order inside a row is missing once
+// the triplets are in their rows, and rows are short. So: count each row's
+// triplets (which also ranks a triplet among its row's), scan the counts, put
+// column and position into the row's place, and sort each row by column and
+// position, 32 rows to a warp in shared memory. Matrices with a row of more
+// than kBucketRow triplets take the radix sort.
+constexpr int kBucketRow = 32;
+constexpr int kBucketWarps = 4;
+constexpr int kBucketBlock = 32 * kBucketWarps;
+
+struct BucketFlags
+{
+   int bad;        // an index outside the matrix
+   int longest;    // triplets of the longest row
+   int duplicate;  // some row has a column twice
+   int pad;
+};
+
+__global__ void __launch_bounds__( 256 )
+coo_count_kernel( int64_t n, const int32_t* __restrict__ ri, const int32_t* __restrict__ ci, int32_t rows, int32_t cols,
+                  unsigned long long* __restrict__ count, int32_t* __restrict__ rank, BucketFlags* F )
+{
+   int most = 0;
+   for( int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x ) {
+      const int32_t r = ri[ i ], c = ci[ i ];
+      if( r < 0 || r >= rows || c < 0 || c >= cols ) {
+         F->bad = 1;
+         continue;
+      }
+      const int k = (int) atomicAdd( count + r, 1ull );
+      rank[ i ] = k;
+      most = max( most, k + 1 );
+   }
+   most = __reduce_max_sync( 0xffffffffu, most );
+   if( ( threadIdx.x & 31 ) == 0 && most > *(volatile int*) &F->longest )
+      atomicMax( &F->longest, most );
+}
+
+__global__ void
+coo_bucket_kernel( int64_t n, const int32_t* __restrict__ ri, const int32_t* __restrict__ ci,
+                   const int64_t* __restrict__ off, const int32_t* __restrict__ rank, uint64_t* __restrict__ keys )
+{
+   for( int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x )
+      keys[ off[ ri[ i ] ] + rank[ i ] ] = ( (uint64_t) (uint32_t) ci[ i ] << 32 ) | (uint32_t) i;
+}
+
+// 32 rows per warp: their keys in shared memory, a lane sorts a row; caps: the
+// row's triplets, unique: its distinct columns (64 bits, scanned later)
+__global__ void __launch_bounds__( kBucketBlock )
+coo_sort_rows_kernel( int32_t rows, const int64_t* __restrict__ off, uint64_t* __restrict__ keys,
+                      int32_t* __restrict__ caps, int32_t* __restrict__ off32, int64_t* __restrict__ unique,
+                      BucketFlags* F )
+{
+   __shared__ uint64_t sh[ kBucketWarps ][ 32 * kBucketRow ];
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+   uint64_t* k = sh[ warp ];
+   const int64_t step = (int64_t) gridDim.x * kBucketBlock;
+   for( int64_t r0 = (int64_t) blockIdx.x * kBucketBlock + 32 * warp; r0 < rows; r0 += step ) {
+      const int64_t r = r0 + lane;
+      const int64_t b = off[ min( r, (int64_t) rows ) ], e = off[ min( r + 1, (int64_t) rows ) ];
+      const int64_t base = __shfl_sync( 0xffffffffu, b, 0 ), end = __shfl_sync( 0xffffffffu, e, 31 );
+      const int total = (int) ( end - base );
+      for( int q = lane; q < total; q += 32 )
+         k[ q ] = keys[ base + q ];
+      __syncwarp();
+      const int lo = (int) ( b - base ), len = (int) ( e - b );
+      int distinct = len > 0 ? 1 : 0;
+      for( int i = 1; i < len; i++ ) {
+         const uint64_t v = k[ lo + i ];
+         int j = i;
+         for( ; j > 0 && k[ lo + j - 1 ] > v; j-- )
+            k[ lo + j ] = k[ lo + j - 1 ];
+         k[ lo + j ] = v;
+      }
+      for( int i = 1; i < len; i++ )
+         distinct += ( k[ lo + i ] >> 32 ) != ( k[ lo + i - 1 ] >> 32 );
+      __syncwarp();
+      for( int q = lane; q < total; q += 32 )
+         keys[ base + q ] = k[ q ];
+      __syncwarp();
+      if( r < rows ) {
+         caps[ r ] = len;
+         off32[ r ] = (int32_t) b;
+         unique[ r ] = distinct;
+         if( distinct != len )
+            F->duplicate = 1;
+      }
+      if( r == rows - 1 ) {
+         off32[ rows ] = (int32_t) e;
+         unique[ rows ] = 0;
+      }
+   }
+}
+
+// no column twice: an element per triplet
+template< typename Real, typename Tin >
+__global__ void
+coo_place_kernel( int64_t n, const uint64_t* __restrict__ keys, const Tin* __restrict__ vals,
+                  int32_t* __restrict__ out_col, Real* __restrict__ out_val )
+{
+   for( int64_t k = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; k < n; k += (int64_t) gridDim.x * blockDim.x ) {
+      const uint64_t key = keys[ k ];
+      out_col[ k ] = (int32_t) ( key >> 32 );
+      out_val[ k ] = (Real) vals[ (uint32_t) key ];
+   }
+}
+
+// a thread per row: runs of one column merged in input order (coo_merge_kernel's arithmetic)
+template< typename Real, typename Tin >
+__global__ void
+coo_merge_rows_kernel( int32_t rows, const int32_t* __restrict__ caps, const int32_t* __restrict__ off,
+                       const int64_t* __restrict__ uoff, const uint64_t* __restrict__ keys, const Tin* __restrict__ vals,
+                       int add, int32_t* __restrict__ out_col, Real* __restrict__ out_val )
+{
+   for( int64_t r = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; r < rows; r += (int64_t) gridDim.x * blockDim.x ) {
+      const int64_t b = off[ r ], e = b + caps[ r ];
+      int64_t u = uoff[ r ];
+      for( int64_t k = b; k < e; ) {
+         const uint32_t c = (uint32_t) ( keys[ k ] >> 32 );
+         Real v = (Real) vals[ (uint32_t) keys[ k ] ];
+         for( k++; k < e && (uint32_t) ( keys[ k ] >> 32 ) == c; k++ ) {
+            const Real nv = (Real) vals[ (uint32_t) keys[ k ] ];
+            v = add ? Real( 1 ) * v + nv : Real( 0 ) * v + nv;
+         }
+         out_col[ u ] = (int32_t) c;
+         out_val[ u ] = v;
+         u++;
+      }
+   }
+}
+
+// consecutive pieces of one allocation, each on a 256-byte boundary
+struct Pieces
+{
+   DevBuf buf;
+   size_t used = 0;
+   template< typename T >
+   size_t add( size_t count )
+   {
+      const size_t at = used;
+      used += ( count * sizeof( T ) + 511 ) / 256 * 256;
+      return at;
+   }
+   template< typename T >
+   T* at( size_t offset ) const
+   {
+      return reinterpret_cast< T* >( static_cast< char* >( buf.p ) + offset );
+   }
+};
+
 static int
 bits_for( int64_t v )  // bits needed for values in [0, v)
 {
@@ -283,12 +436,104 @@ bits_for( int64_t v )  // bits needed for values in [0, v)
    return b;
 }
 
+// setRowCapacities( caps ): every row's `used` elements must fit; total: the
+// sum of the capacities
+static b2s_status
+user_capacities( const int32_t* caps, const int32_t* used, int32_t rows, int64_t& total, cudaStream_t s )
+{
+   DevBuf c64, badf;
+   B2S_TRY( c64.alloc( ( (size_t) rows + 1 ) * sizeof( int64_t ) ) );
+   B2S_TRY( badf.alloc( sizeof( int ) ) );
+   const int none = INT32_MAX;
+   B2S_TRY( copy_h2d( badf.p, &none, sizeof( int ), s ) );
+   caps_check_kernel<<< grid_of( (int64_t) rows + 1 ), 256, 0, s >>>( caps, used, rows, c64.as< int64_t >(), badf.as< int >() );
+   B2S_TRY_CUDA( cudaGetLastError() );
+   int badrow = INT32_MAX;
+   B2S_TRY( copy_d2h( &badrow, badf.p, sizeof( int ), s ) );
+   if( badrow != INT32_MAX ) {
+      set_error( "The capacity of the sparse matrix row number %d was exceeded.", badrow );
+      return B2S_INVALID_ARG;
+   }
+   B2S_TRY( scan_exclusive_i64( c64.as< int64_t >(), (int64_t) rows + 1, s ) );
+   return copy_d2h( &total, c64.as< int64_t >() + rows, sizeof( int64_t ), s );
+}
+
+// The row-bucket assembly; taken = false (and nothing built) when a row is too
+// long for it.
+template< typename Real, typename Tin >
+static b2s_status
+assemble_rows( b2s_format format, b2s_dtype dtype, int32_t rows, int32_t cols, int64_t n, const int32_t* ri,
+               const int32_t* ci, const Tin* vals, int add, const int32_t* caps_user, const b2s_matrix_opts& o,
+               cudaStream_t s, b2s_matrix* out, bool& taken )
+{
+   taken = false;
+   if( n == 0 || rows == 0 || n > INT32_MAX )
+      return B2S_OK;
+   const size_t m = (size_t) rows + 1;
+   Pieces W;
+   const size_t p_off = W.add< int64_t >( m ), p_rank = W.add< int32_t >( n ), p_flags = W.add< BucketFlags >( 1 ),
+                p_keys = W.add< uint64_t >( n ), p_caps = W.add< int32_t >( m ), p_off32 = W.add< int32_t >( m ),
+                p_unique = W.add< int64_t >( m ), p_col = W.add< int32_t >( n ), p_val = W.add< Real >( n ),
+                p_used = W.add< int32_t >( caps_user ? m : 0 );
+   B2S_TRY( W.buf.alloc( W.used ) );
+   int64_t *off = W.at< int64_t >( p_off ), *unique = W.at< int64_t >( p_unique );
+   int32_t *rank = W.at< int32_t >( p_rank ), *caps = W.at< int32_t >( p_caps ), *off32 = W.at< int32_t >( p_off32 ),
+           *ucol = W.at< int32_t >( p_col );
+   uint64_t* keys = W.at< uint64_t >( p_keys );
+   Real* uval = W.at< Real >( p_val );
+   BucketFlags* F = W.at< BucketFlags >( p_flags );
+   B2S_TRY_CUDA( cudaMemsetAsync( off, 0, m * sizeof( int64_t ), s ) );
+   B2S_TRY_CUDA( cudaMemsetAsync( F, 0, sizeof( BucketFlags ), s ) );
+   coo_count_kernel<<< grid_of( n ), 256, 0, s >>>( n, ri, ci, rows, cols, reinterpret_cast< unsigned long long* >( off ),
+                                                    rank, F );
+   B2S_TRY_CUDA( cudaGetLastError() );
+   BucketFlags h{};
+   B2S_TRY( copy_d2h( &h, F, sizeof( h ), s ) );
+   if( h.bad ) {
+      set_error( "triplet index outside the %d x %d matrix", rows, cols );
+      return B2S_INVALID_ARG;
+   }
+   if( h.longest > kBucketRow )
+      return B2S_OK;
+   B2S_TRY( scan_exclusive_i64( off, (int64_t) m, s ) );
+   coo_bucket_kernel<<< grid_of( n ), 256, 0, s >>>( n, ri, ci, off, rank, keys );
+   coo_sort_rows_kernel<<< grid_of( rows, kBucketBlock ), kBucketBlock, 0, s >>>( rows, off, keys, caps, off32, unique, F );
+   B2S_TRY_CUDA( cudaGetLastError() );
+   B2S_TRY( copy_d2h( &h, F, sizeof( h ), s ) );
+   int64_t nu = n, caps_total = n;
+   const int32_t* caps_used = caps;
+   if( ! h.duplicate && ! caps_user ) {
+      coo_place_kernel< Real, Tin ><<< grid_of( n ), 256, 0, s >>>( n, keys, vals, ucol, uval );
+      B2S_TRY_CUDA( cudaGetLastError() );
+   }
+   else {
+      if( caps_user ) {
+         int32_t* used = W.at< int32_t >( p_used );
+         i64_to_i32_kernel<<< grid_of( (int64_t) m ), 256, 0, s >>>( unique, (int64_t) m, used );
+         B2S_TRY( user_capacities( caps_user, used, rows, caps_total, s ) );
+         caps_used = caps_user;
+      }
+      B2S_TRY( scan_exclusive_i64( unique, (int64_t) m, s ) );
+      B2S_TRY( copy_d2h( &nu, unique + rows, sizeof( int64_t ), s ) );
+      coo_merge_rows_kernel< Real, Tin ><<< grid_of( rows ), 256, 0, s >>>( rows, caps, off32, unique, keys, vals, add,
+                                                                         ucol, uval );
+      i64_to_i32_kernel<<< grid_of( (int64_t) m ), 256, 0, s >>>( unique, (int64_t) m, off32 );
+      B2S_TRY_CUDA( cudaGetLastError() );
+   }
+   taken = true;
+   return matrix_from_assembled( format, dtype, rows, cols, nu, off32, ucol, uval, caps_used, caps_total, o, s, out );
+}
+
 template< typename Real, typename Tin >
 static b2s_status
 assemble( b2s_format format, b2s_dtype dtype, int32_t rows, int32_t cols, int64_t n, const int32_t* ri,
           const int32_t* ci, const Tin* vals, int add, const int32_t* caps_user, const b2s_matrix_opts& o,
           cudaStream_t s, b2s_matrix* out )
 {
+   bool taken = false;
+   B2S_TRY( ( assemble_rows< Real, Tin >( format, dtype, rows, cols, n, ri, ci, vals, add, caps_user, o, s, out, taken ) ) );
+   if( taken )
+      return B2S_OK;
    const int cbits = bits_for( cols ), rbits = bits_for( rows );
    DevBuf keys, idx, keys2, idx2, flag;
    B2S_TRY( keys.alloc( (size_t) std::max< int64_t >( n, 1 ) * sizeof( uint64_t ) ) );
@@ -359,23 +604,7 @@ assemble( b2s_format format, b2s_dtype dtype, int32_t rows, int32_t cols, int64_
    int64_t caps_total = n;
    const int32_t* caps_used = caps.as< int32_t >();
    if( caps_user ) {
-      // setRowCapacities( caps ): check that every row's elements fit, sum the capacities
-      DevBuf c64, badf;
-      B2S_TRY( c64.alloc( ( (size_t) rows + 1 ) * sizeof( int64_t ) ) );
-      B2S_TRY( badf.alloc( sizeof( int ) ) );
-      const int none = INT32_MAX;
-      B2S_TRY( copy_h2d( badf.p, &none, sizeof( int ), s ) );
-      caps_check_kernel<<< grid_of( (int64_t) rows + 1 ), 256, 0, s >>>( caps_user, rcount.as< int32_t >(), rows,
-                                                                         c64.as< int64_t >(), badf.as< int >() );
-      B2S_TRY_CUDA( cudaGetLastError() );
-      int badrow = INT32_MAX;
-      B2S_TRY( copy_d2h( &badrow, badf.p, sizeof( int ), s ) );
-      if( badrow != INT32_MAX ) {
-         set_error( "The capacity of the sparse matrix row number %d was exceeded.", badrow );
-         return B2S_INVALID_ARG;
-      }
-      B2S_TRY( scan_exclusive_i64( c64.as< int64_t >(), (int64_t) rows + 1, s ) );
-      B2S_TRY( copy_d2h( &caps_total, c64.as< int64_t >() + rows, sizeof( int64_t ), s ) );
+      B2S_TRY( user_capacities( caps_user, rcount.as< int32_t >(), rows, caps_total, s ) );
       caps_used = caps_user;
    }
    return matrix_from_assembled( format, dtype, rows, cols, nu, off.as< int32_t >(), ucol.as< int32_t >(), uval.p,
