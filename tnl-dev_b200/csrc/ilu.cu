@@ -43,6 +43,131 @@ grid_n( int64_t n )
    return (int) std::max< int64_t >( 1, std::min< int64_t >( ( n + 255 ) / 256, (int64_t) num_sms() * 32 ) );
 }
 
+// Blocks of the substitutions, or none when the rows do not suit a lane per
+// row. A step across blocks goes through L2, one inside a block through shared
+// memory, so blocks are large; but a block's warps share one SM. Measured with
+// 2,048 / 8,192 / 16,384 rows at least: 32^3 stencil 155 / 132 / 170 us, 64^3
+// 321 / 284 / 256 us, 2D 140^2 285 / 234 / 228 us.
+// A lane walks its row alone: rows of up to kTrsvMeanRow factor entries on
+// average, none longer than kTrsvMaxRow.
+constexpr int32_t kTrsvRows = 8192;
+constexpr int32_t kTrsvMeanRow = 24, kTrsvMaxRow = 128;
+
+template< typename Real >
+static void
+choose_blocks( IluFactors< Real >& F, const std::vector< int32_t >& hoff )
+{
+   F.blocks = 0;
+   const int32_t n = F.n;
+   if( n == 0 )
+      return;
+   int32_t longest = 0;
+   for( int32_t i = 0; i < n; i++ )
+      longest = std::max( longest, hoff[ i + 1 ] - hoff[ i ] );
+   if( longest > kTrsvMaxRow || (int64_t) hoff[ n ] > (int64_t) kTrsvMeanRow * n )
+      return;
+   const int32_t want = std::max( 1, std::min( num_sms(), ( n + kTrsvRows - 1 ) / kTrsvRows ) );
+   const int32_t rows = ( n + want - 1 ) / want;
+   if( (int64_t) rows * (int64_t) sizeof( Real ) > kTrsvSmemMax )
+      return;  // x of a block has to fit in shared memory
+   F.rows_per_block = rows;
+   F.blocks = ( n + rows - 1 ) / rows;
+}
+
+// One triangle's batches: the rows of each block by level, cut into batches of
+// up to 32 rows of one level. deps( i ): row i's entries in this triangle.
+template< typename Real, class Deps >
+static b2s_status
+block_plan( IluFactors< Real >& F, TrsvPlan< Real >& P, const std::vector< int32_t >& lev, Deps deps, cudaStream_t s )
+{
+   const int32_t G = F.blocks, R = F.rows_per_block;
+   std::vector< int32_t > first( (size_t) G + 1, 0 ), row, width, order, count;
+   row.reserve( (size_t) F.n + (size_t) F.n / 4 );
+   for( int32_t c = 0; c < G; c++ ) {
+      const int32_t r0 = c * R, r1 = std::min( F.n, r0 + R );
+      const auto range = std::minmax_element( lev.begin() + r0, lev.begin() + r1 );
+      const int32_t lo = *range.first;
+      const int64_t span = (int64_t) *range.second - lo + 1;
+      // the block's rows by level, in increasing order within one
+      order.resize( (size_t) ( r1 - r0 ) );
+      if( span <= 8LL * R ) {
+         count.assign( (size_t) span + 1, 0 );
+         for( int32_t i = r0; i < r1; i++ )
+            count[ lev[ i ] - lo + 1 ]++;
+         for( int64_t l = 0; l < span; l++ )
+            count[ l + 1 ] += count[ l ];
+         for( int32_t i = r0; i < r1; i++ )
+            order[ count[ lev[ i ] - lo ]++ ] = i;
+      }
+      else {
+         for( int32_t i = r0; i < r1; i++ )
+            order[ i - r0 ] = i;
+         std::stable_sort( order.begin(), order.end(), [ & ]( int32_t x, int32_t y ) { return lev[ x ] < lev[ y ]; } );
+      }
+      int32_t fill = 32, level = -1;
+      for( const int32_t i : order ) {
+         if( fill == 32 || level != lev[ i ] ) {
+            row.resize( width.size() * 32, -1 );
+            width.push_back( 0 );
+            fill = 0;
+            level = lev[ i ];
+         }
+         row.push_back( i );
+         fill++;
+         width.back() = std::max( width.back(), deps( i ) );
+      }
+      row.resize( width.size() * 32, -1 );
+      first[ c + 1 ] = (int32_t) width.size();
+   }
+   P.batches = first[ G ];
+   width.push_back( 0 );
+   int64_t slots = 0;
+   for( int32_t q = 0; q <= P.batches; q++ ) {
+      const int32_t w = width[ q ];
+      width[ q ] = (int32_t) slots;
+      slots += w;
+   }
+   if( slots > INT32_MAX / 64 ) {  // padded slots past int32: warp per row
+      F.blocks = 0;
+      return B2S_OK;
+   }
+   B2S_TRY( P.bfirst.alloc( first.size() * sizeof( int32_t ) ) );
+   B2S_TRY( P.bptr.alloc( width.size() * sizeof( int32_t ) ) );
+   B2S_TRY( P.row.alloc( row.size() * sizeof( int32_t ) ) );
+   B2S_TRY( P.len.alloc( row.size() * sizeof( int32_t ) ) );
+   B2S_TRY( P.dg.alloc( row.size() * sizeof( Real ) ) );
+   B2S_TRY( P.col.alloc( (size_t) std::max< int64_t >( slots, 1 ) * 32 * sizeof( int32_t ) ) );
+   B2S_TRY( P.val.alloc( (size_t) std::max< int64_t >( slots, 1 ) * 32 * sizeof( Real ) ) );
+   B2S_TRY( copy_h2d( P.bfirst.p, first.data(), first.size() * sizeof( int32_t ), s ) );
+   B2S_TRY( copy_h2d( P.bptr.p, width.data(), width.size() * sizeof( int32_t ), s ) );
+   return copy_h2d( P.row.p, row.data(), row.size() * sizeof( int32_t ), s );
+}
+
+template< typename Real >
+b2s_status
+ilu_pack( IluFactors< Real >& F, cudaStream_t s )
+{
+   if( F.blocks == 0 )
+      return B2S_OK;
+   B2S_TRY( F.yz.alloc( 2 * (size_t) F.n * sizeof( Real ) ) );
+   B2S_TRY( F.clear_scratch( s ) );
+   const TrsvPlan< Real >&l = F.plan_l, &u = F.plan_u;
+   trsv_pack_kernel< Real, false ><<< grid_n( 32LL * l.batches ), 256, 0, s >>>(
+      32 * l.batches, l.row.template as< int32_t >(), l.bptr.template as< int32_t >(), F.off,
+      F.diag.template as< int32_t >(), F.col, F.lu.template as< Real >(), l.len.template as< int32_t >(),
+      l.col.template as< int32_t >(), l.val.template as< Real >(), l.dg.template as< Real >() );
+   trsv_pack_kernel< Real, true ><<< grid_n( 32LL * u.batches ), 256, 0, s >>>(
+      32 * u.batches, u.row.template as< int32_t >(), u.bptr.template as< int32_t >(), F.off,
+      F.diag.template as< int32_t >(), F.col, F.lu.template as< Real >(), u.len.template as< int32_t >(),
+      u.col.template as< int32_t >(), u.val.template as< Real >(), u.dg.template as< Real >() );
+   B2S_TRY_CUDA( cudaGetLastError() );
+   B2S_TRY_CUDA( cudaMemsetAsync( F.state.p, 0, sizeof( unsigned int ), s ) );  // the block tickets
+   return B2S_OK;
+}
+
+template b2s_status ilu_pack< double >( IluFactors< double >&, cudaStream_t );
+template b2s_status ilu_pack< float >( IluFactors< float >&, cudaStream_t );
+
 template< typename Real >
 b2s_status
 ilu_levels( IluFactors< Real >& F, const std::vector< int32_t >& hoff, const std::vector< int32_t >& hcol,
@@ -50,6 +175,7 @@ ilu_levels( IluFactors< Real >& F, const std::vector< int32_t >& hoff, const std
 {
    const int32_t n = F.n;
    std::vector< int32_t > lev( (size_t) std::max( n, 1 ) ), ord;
+   choose_blocks( F, hoff );
    auto order = [ & ]( int depth, DevBuf& out, int32_t& len ) -> b2s_status
    {
       // counting sort of the rows by level, rows in increasing order within a
@@ -70,6 +196,7 @@ ilu_levels( IluFactors< Real >& F, const std::vector< int32_t >& hoff, const std
       B2S_TRY( out.alloc( ord.size() * sizeof( int32_t ) ) );
       return copy_h2d( out.p, ord.data(), ord.size() * sizeof( int32_t ), s );
    };
+   ord.reserve( (size_t) n + 32 );
    int depth = 0;
    for( int32_t i = 0; i < n; i++ ) {
       int l = 0;
@@ -80,6 +207,8 @@ ilu_levels( IluFactors< Real >& F, const std::vector< int32_t >& hoff, const std
    }
    F.levels_l = depth;
    B2S_TRY( order( depth, F.ord_l, F.n_ord_l ) );
+   if( F.blocks > 0 )
+      B2S_TRY( block_plan< Real >( F, F.plan_l, lev, [ & ]( int32_t i ) { return hdiag[ i ] - hoff[ i ]; }, s ) );
    depth = 0;
    for( int32_t i = n - 1; i >= 0; i-- ) {
       int l = 0;
@@ -89,7 +218,10 @@ ilu_levels( IluFactors< Real >& F, const std::vector< int32_t >& hoff, const std
       depth = std::max( depth, l + 1 );
    }
    F.levels_u = depth;
-   B2S_TRY( order( depth, F.ord_u, F.n_ord_u ) );
+   if( F.blocks > 0 )
+      B2S_TRY( block_plan< Real >( F, F.plan_u, lev, [ & ]( int32_t i ) { return hoff[ i + 1 ] - hdiag[ i ] - 1; }, s ) );
+   if( F.blocks == 0 )  // U's order serves the warp-per-row kernel only (L's the factorization too)
+      B2S_TRY( order( depth, F.ord_u, F.n_ord_u ) );
    // resident warps only: every SM full of 256-thread blocks
    F.grid = num_sms() * ( 2048 / kIluBlock );
    return B2S_OK;
@@ -178,6 +310,7 @@ ilu_factorize( const b2s_matrix_t* A, const Real* values, IluFactors< Real >& F,
    ilu_begin_kernel< NoGate ><<< 1, 1, 0, s >>>( v.st, NoGate{} );
    ilu_factor_kernel< Real ><<< F.grid, kIluBlock, 0, s >>>( v );
    B2S_TRY_CUDA( cudaGetLastError() );
+   B2S_TRY( ilu_pack( F, s ) );
    B2S_TRY_CUDA( cudaStreamSynchronize( s ) );
    return F.check( s );
 }

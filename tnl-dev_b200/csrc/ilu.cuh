@@ -17,6 +17,9 @@
 // raises the error word and returns, and the others leave as soon as they see
 // it; the host turns the word into B2S_TIMEOUT.
 //
+// The substitutions of factors with short rows run by blocks of rows instead
+// (ilu_block_trsv_kernel).
+//
 // Arithmetic follows TNL's loops element by element: for row i and each of
 // its L entries k in increasing order, L_ik = L_ik / U_kk and every later
 // entry j of the row takes L_ik * U_kj off (U_kj = 0 when absent); the
@@ -41,10 +44,10 @@ constexpr int kIluSpinLimit = 1 << 21;
 
 struct IluState
 {
-   unsigned int ticket;  // next row to claim
+   unsigned int ticket;  // next row (warp-per-row kernels) or block of rows to claim
    int epoch;            // the current pass; a row is done when its flag equals it
    int error;            // 1: a bounded wait gave up
-   int pad;
+   int skip;             // the current pass is gated off
 };
 
 template< typename Real >
@@ -122,12 +125,14 @@ ilu_wait( const int32_t* flag, int epoch, IluState* st )
    return false;
 }
 
-// a new pass: tickets from 0, a fresh epoch
+// a new pass of the warp-per-row kernels: tickets from 0, a fresh epoch
 template< class Gate >
 __global__ void
 ilu_begin_kernel( IluState* st, Gate gate )
 {
-   if( gate.skip() )
+   const bool off = gate.skip();
+   st->skip = off ? 1 : 0;
+   if( off )
       return;
    st->ticket = 0;
    st->epoch += 1;
@@ -197,14 +202,15 @@ ilu_factor_kernel( IluView< Real > L )
 // parallel; the sum runs in TNL's order through shuffles); x may be b.
 // PLAIN: every term a rounded product subtracted in order (the ILUT
 // substitutions, whose loops the reference build does not vectorize).
-template< typename Real, bool UPPER, class Gate, bool PLAIN = false >
+// Serves factors whose rows are long or too many for the block kernel below.
+template< typename Real, bool UPPER, bool PLAIN = false >
 __global__ void __launch_bounds__( kIluBlock )
-ilu_trsv_kernel( IluView< Real > L, const Real* b, Real* x, Gate gate )
+ilu_trsv_kernel( IluView< Real > L, const Real* b, Real* x )
 {
-   if( gate.skip() )
-      return;
    const int lane = threadIdx.x & 31;
    IluState* st = L.st;
+   if( *(volatile int*) &st->skip )
+      return;
    const int epoch = *(volatile int*) &st->epoch;
    const int32_t* ord = UPPER ? L.ord_u : L.ord_l;
    const int32_t nord = UPPER ? L.n_u : L.n_l;
@@ -251,6 +257,346 @@ ilu_trsv_kernel( IluView< Real > L, const Real* b, Real* x, Gate gate )
    }
 }
 
+// ---------------------------------------------------------------------------
+// Substitutions by blocks of rows (short rows: stencils and the like).
+//
+// A substitution is a chain of as many steps as there are levels, so its time
+// is the latency of one step. The warp-per-row kernel above pays a flag poll,
+// a load of x, a fence and a flag store through L2 for every step: 4.9 us per
+// level measured on a 128^3 stencil. Here a CTA owns a contiguous block of
+// rows and keeps their x in shared memory; most of a stencil row's
+// dependencies are in its own block, so most steps of the chain are a store
+// and a poll of shared memory.
+//   * The rows of a block are ordered by level and cut into batches of at most
+//     32 rows of one level, a lane per row (so no lane waits for another of
+//     its warp); warp w takes batches w, w + warps, ... of its block in order.
+//   * A value is its own flag, in shared memory for the block's rows and in L2
+//     for the others': it starts as a signalling NaN that no operation
+//     returns, and whoever needs it looks again until it is there. So a step
+//     needs no fence: one would wait for the loads ahead that are in flight
+//     (with a fence, a flag or a count per batch: 1,200 cycles per step). A
+//     computed value with those bits (copied through from b) is stored as the
+//     quiet NaN. A warp that is early looks at one word of shared memory, not
+//     at all of its rows', which would keep the load pipe from the warp whose
+//     turn it is. The first look at other blocks' rows goes out before that.
+//   * A batch's columns, values and diagonal are stored batch by batch in slot
+//     order, so a warp loads them coalesced, one and two batches ahead of the
+//     one whose turn it is.
+//   * Blocks are claimed in dependency order from a ticket counter: a claimed
+//     block waits only for blocks claimed before it, whose CTAs are running.
+//     The CTA that takes the last ticket puts the counter back.
+//   * Both passes publish in their own scratch vector (y: L^-1 b, z: U^-1 y);
+//     each pass puts the other's scratch back to the signalling NaN for the
+//     next application, so there is no pass to clear them, and b may be x.
+// Every wait is bounded as above (the limits are longer: a block may wait for
+// all blocks before it). Rows per block: see choose_blocks.
+// Measured, both substitutions of one application through the public call
+// (warp per row before): 3D stencils 10^3 177 -> 52 us, 32^3 535 -> 132 us,
+// 64^3 1,106 -> 284 us, 128^3 3,748 -> 1,009 us; 2D 140^2 1,233 -> 234 us.
+constexpr int kTrsvBlock = 256;                // 128 to 512 measured alike
+constexpr int kTrsvWarps = kTrsvBlock / 32;
+constexpr int kTrsvSlots = 4;                  // slots of the next batch loaded ahead
+constexpr int kTrsvSmemMax = 200 * 1024;       // x of one block in shared memory
+constexpr int kTrsvSpinLocal = 1 << 26;        // polls of shared memory (a few seconds)
+constexpr int kTrsvSpinRemote = 1 << 23;       // polls of L2 (about 2 s)
+
+template< typename Real >
+struct TrsvBits;
+template<>
+struct TrsvBits< double >
+{
+   using type = unsigned long long;
+   static constexpr type pending = 0xFFF3B25D5EA10F0Full, quiet = 1ull << 51;
+};
+template<>
+struct TrsvBits< float >
+{
+   using type = unsigned int;
+   static constexpr type pending = 0xFFB1D5EAu, quiet = 1u << 22;
+};
+__device__ __forceinline__ unsigned long long
+trsv_bits( double v )
+{
+   return (unsigned long long) __double_as_longlong( v );
+}
+__device__ __forceinline__ unsigned int
+trsv_bits( float v )
+{
+   return __float_as_uint( v );
+}
+__device__ __forceinline__ double
+trsv_value( unsigned long long b )
+{
+   return __longlong_as_double( (long long) b );
+}
+__device__ __forceinline__ float
+trsv_value( unsigned int b )
+{
+   return __uint_as_float( b );
+}
+__device__ __forceinline__ unsigned long long
+trsv_ld_remote( const unsigned long long* p )
+{
+   unsigned long long v;
+   asm volatile( "ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"( v ) : "l"( p ) : "memory" );
+   return v;
+}
+__device__ __forceinline__ unsigned int
+trsv_ld_remote( const unsigned int* p )
+{
+   unsigned int v;
+   asm volatile( "ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"( v ) : "l"( p ) : "memory" );
+   return v;
+}
+__device__ __forceinline__ void
+trsv_st_remote( unsigned long long* p, unsigned long long v )
+{
+   asm volatile( "st.relaxed.gpu.global.b64 [%0], %1;" ::"l"( p ), "l"( v ) : "memory" );
+}
+__device__ __forceinline__ void
+trsv_st_remote( unsigned int* p, unsigned int v )
+{
+   asm volatile( "st.relaxed.gpu.global.b32 [%0], %1;" ::"l"( p ), "r"( v ) : "memory" );
+}
+
+// one triangle's rows in block and batch order
+template< typename Real >
+struct TrsvView
+{
+   int32_t n, rows_per_block;
+   const int32_t* bfirst;  // first batch of each block (blocks + 1 entries)
+   const int32_t* bptr;    // first slot of each batch / 32 (batches + 1 entries)
+   const int32_t* row;     // row of each lane of each batch, -1: none
+   const int32_t* len;     // its dependencies
+   const int32_t* col;     // slot k of lane l of a batch at ( bptr + k ) * 32 + l
+   const Real* val;
+   const Real* dg;         // U_ii of each lane of each batch (upper only)
+};
+
+template< typename Real, bool UPPER, bool PLAIN, class Gate >
+__global__ void __launch_bounds__( kTrsvBlock, 1 )
+ilu_block_trsv_kernel( TrsvView< Real > T, IluState* st, const Real* b, typename TrsvBits< Real >::type* pub,
+                       typename TrsvBits< Real >::type* other, Real* x, Gate gate )
+{
+   using Bits = typename TrsvBits< Real >::type;
+   constexpr Bits pending = TrsvBits< Real >::pending;
+   extern __shared__ __align__( 16 ) unsigned char trsv_smem[];
+   Bits* xs = reinterpret_cast< Bits* >( trsv_smem );
+   __shared__ int s_block;
+   if( gate.skip() )
+      return;
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+   if( threadIdx.x == 0 ) {
+      const unsigned t = atomicAdd( &st->ticket, 1u );
+      if( t == gridDim.x - 1 )
+         atomicExch( &st->ticket, 0u );
+      s_block = UPPER ? (int) ( gridDim.x - 1 - t ) : (int) t;
+   }
+   __syncthreads();
+   const int blk = s_block;
+   const int c0 = blk * T.rows_per_block, c1 = min( T.n, c0 + T.rows_per_block );
+   for( int i = threadIdx.x; i < c1 - c0; i += kTrsvBlock ) {
+      xs[ i ] = pending;
+      if( ! UPPER )
+         other[ c0 + i ] = pending;
+   }
+   __syncthreads();
+   const int last = T.bfirst[ blk + 1 ];
+   bool ok = true;  // false once a wait gave up: no more waits, the count goes on
+   // a batch's lane: loaded two batches (meta) and one batch (slots, right-hand
+   // side) ahead of its turn, so that no turn waits for them
+   struct Meta
+   {
+      int row, len, ptr, width;
+      Real dg;
+   };
+   struct Slots
+   {
+      Real b, val[ kTrsvSlots ];
+      int col[ kTrsvSlots ];
+   };
+   auto load_meta = [ & ]( int q )
+   {
+      Meta m{ -1, 0, 0, 0, Real( 1 ) };
+      if( q < last ) {
+         m.ptr = __ldg( T.bptr + q );
+         m.width = __ldg( T.bptr + q + 1 );
+         m.row = __ldg( T.row + 32 * (int64_t) q + lane );
+         m.len = __ldg( T.len + 32 * (int64_t) q + lane );
+         if( UPPER )
+            m.dg = __ldg( T.dg + 32 * (int64_t) q + lane );
+      }
+      return m;
+   };
+   auto load_slots = [ & ]( const Meta& m, int k0, Slots& s )
+   {
+      const int64_t g = 32 * (int64_t) ( m.ptr + k0 ) + lane;
+#pragma unroll
+      for( int k = 0; k < kTrsvSlots; k++ ) {
+         s.col[ k ] = c0;  // no element: a place of this block
+         s.val[ k ] = 0;
+         if( k0 + k < m.len ) {
+            s.col[ k ] = __ldg( T.col + g + 32 * k );
+            s.val[ k ] = __ldg( T.val + g + 32 * k );
+         }
+      }
+   };
+   int q = T.bfirst[ blk ] + warp;
+   Meta next = load_meta( q ), after = load_meta( q + kTrsvWarps );
+   Slots ahead;
+   auto load_ahead = [ & ]()
+   {
+      load_slots( next, 0, ahead );
+      ahead.b = next.row >= 0 ? __ldcg( b + next.row ) : Real( 0 );
+   };
+   load_ahead();
+   for( ; q < last; q += kTrsvWarps ) {
+      const Meta m = next;
+      Slots s = ahead;
+      const int width = m.width - m.ptr;
+      Real acc = s.b;
+      // where the slots' values are: in xs, or (at < 0) in another block's,
+      // whose first look goes out now
+      Bits xr[ kTrsvSlots ];
+      int at[ kTrsvSlots ];
+      auto look = [ & ]( int k0 )
+      {
+#pragma unroll
+         for( int k = 0; k < kTrsvSlots; k++ ) {
+            const unsigned i = (unsigned) ( s.col[ k ] - c0 );
+            const bool in = k0 + k < m.len, mine = i < (unsigned) ( c1 - c0 );
+            at[ k ] = in && mine ? (int) i : -1;
+            xr[ k ] = 0;
+            if( in && ! mine )
+               xr[ k ] = trsv_ld_remote( pub + s.col[ k ] );
+         }
+      };
+      look( 0 );
+      next = after;
+      load_ahead();
+      after = load_meta( q + 2 * kTrsvWarps );
+      for( int k0 = 0; k0 < width; k0 += kTrsvSlots ) {
+         if( k0 > 0 ) {
+            load_slots( m, k0, s );
+            look( k0 );
+         }
+         // one value stands for the warp's: while it is missing the warp polls
+         // a single word
+         int some = -1;
+#pragma unroll
+         for( int k = 0; k < kTrsvSlots; k++ )
+            some = max( some, at[ k ] );
+         const unsigned have = __ballot_sync( 0xffffffffu, some >= 0 );
+         if( have ) {
+            some = __shfl_sync( 0xffffffffu, some, __ffs( have ) - 1 );
+            for( int it = 0; *(volatile Bits*) &xs[ some ] == pending && ok; it++ )
+               if( ( it & 1023 ) == 1023 && ( it >= kTrsvSpinLocal || *(volatile int*) &st->error ) )
+                  ok = false;
+         }
+         // The step's latency is what counts from here to the store of x: no
+         // branches that part the warp, loads of shared memory side by side.
+         Bits xv[ kTrsvSlots ];
+         bool wait;
+         int it = 0;
+         do {
+            wait = false;
+#pragma unroll
+            for( int k = 0; k < kTrsvSlots; k++ ) {
+               xv[ k ] = *(volatile Bits*) &xs[ max( at[ k ], 0 ) ];
+               if( xr[ k ] == pending )
+                  xr[ k ] = trsv_ld_remote( pub + s.col[ k ] );
+            }
+#pragma unroll
+            for( int k = 0; k < kTrsvSlots; k++ ) {
+               xv[ k ] = at[ k ] < 0 ? xr[ k ] : xv[ k ];
+               wait = wait || xv[ k ] == pending;
+            }
+            if( ( ++it & 255 ) == 0 && ( it >= kTrsvSpinRemote || *(volatile int*) &st->error ) )
+               ok = false;
+         } while( __any_sync( 0xffffffffu, wait && ok ) );
+#pragma unroll
+         for( int k = 0; k < kTrsvSlots; k++ ) {
+            const Real x_k = trsv_value( xv[ k ] );
+            const Real t = PLAIN ? msub< false >( acc, s.val[ k ], x_k ) : sum_term< Real >( acc, s.val[ k ], x_k, k0 + k, m.len );
+            acc = k0 + k < m.len ? t : acc;
+         }
+      }
+      if( UPPER )
+         acc = acc / m.dg;
+      Bits r = trsv_bits( acc );
+      if( r == pending )
+         r |= TrsvBits< Real >::quiet;
+      if( m.row >= 0 ) {
+         *(volatile Bits*) &xs[ m.row - c0 ] = r;
+         trsv_st_remote( pub + m.row, r );
+         if( UPPER ) {
+            x[ m.row ] = trsv_value( r );
+            other[ m.row ] = pending;  // this pass has read its right-hand side
+         }
+      }
+   }
+   if( ! ok )
+      atomicExch( &st->error, 1 );
+}
+
+// the packed rows of one triangle (slots, lengths, diagonal) from the factors
+template< typename Real, bool UPPER >
+__global__ void
+trsv_pack_kernel( int32_t lanes, const int32_t* __restrict__ row, const int32_t* __restrict__ bptr,
+                  const int32_t* __restrict__ off, const int32_t* __restrict__ diag, const int32_t* __restrict__ col,
+                  const Real* __restrict__ lu, int32_t* __restrict__ len, int32_t* __restrict__ pcol,
+                  Real* __restrict__ pval, Real* __restrict__ dg )
+{
+   for( int64_t t = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; t < lanes; t += (int64_t) gridDim.x * blockDim.x ) {
+      const int i = row[ t ];
+      if( i < 0 ) {
+         len[ t ] = 0;
+         if( UPPER )
+            dg[ t ] = 1;
+         continue;
+      }
+      const int d = diag[ i ];
+      const int b0 = UPPER ? d + 1 : off[ i ], b1 = UPPER ? off[ i + 1 ] : d;
+      const int64_t g = 32 * (int64_t) bptr[ t >> 5 ] + ( t & 31 );
+      for( int k = b0; k < b1; k++ ) {
+         pcol[ g + 32 * (int64_t) ( k - b0 ) ] = col[ k ];
+         pval[ g + 32 * (int64_t) ( k - b0 ) ] = lu[ k ];
+      }
+      len[ t ] = b1 - b0;
+      if( UPPER )
+         dg[ t ] = lu[ d ];
+   }
+}
+
+template< typename Bits >
+__global__ void
+trsv_clear_kernel( Bits* y, int64_t count, Bits v )
+{
+   for( int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < count; i += (int64_t) gridDim.x * blockDim.x )
+      y[ i ] = v;
+}
+
+// One triangle in block and batch order (empty: the warp-per-row kernel runs).
+template< typename Real >
+struct TrsvPlan
+{
+   DevBuf bfirst, bptr, row, len, col, val, dg;
+   int32_t batches = 0;
+
+   TrsvView< Real > view( int32_t n, int32_t rows_per_block ) const
+   {
+      return TrsvView< Real >{ n,
+                               rows_per_block,
+                               bfirst.as< int32_t >(),
+                               bptr.as< int32_t >(),
+                               row.as< int32_t >(),
+                               len.as< int32_t >(),
+                               col.as< int32_t >(),
+                               val.as< Real >(),
+                               dg.as< Real >() };
+   }
+};
+
 // The factors of one matrix in one value type, with their pass state.
 template< typename Real >
 struct IluFactors
@@ -264,6 +610,10 @@ struct IluFactors
    int levels_l = 0, levels_u = 0;  // depth of the dependency chains
    int32_t n_ord_l = 0, n_ord_u = 0;
    bool plain_sum = false;  // ILUT factors: substitution terms subtracted one by one
+   // substitutions by blocks of rows (blocks == 0: warp per row)
+   TrsvPlan< Real > plan_l, plan_u;
+   DevBuf yz;  // the two passes' scratch vectors
+   int32_t blocks = 0, rows_per_block = 0;
 
    IluView< Real > view() const
    {
@@ -277,17 +627,44 @@ struct IluFactors
    {
       if( n == 0 )
          return B2S_OK;
+      if( blocks > 0 )
+         return plain_sum ? apply_blocks< true >( b, x, s, gate ) : apply_blocks< false >( b, x, s, gate );
       const IluView< Real > v = view();
       ilu_begin_kernel< Gate ><<< 1, 1, 0, s >>>( v.st, gate );
       if( plain_sum )
-         ilu_trsv_kernel< Real, false, Gate, true ><<< grid, kIluBlock, 0, s >>>( v, b, x, gate );
+         ilu_trsv_kernel< Real, false, true ><<< grid, kIluBlock, 0, s >>>( v, b, x );
       else
-         ilu_trsv_kernel< Real, false, Gate ><<< grid, kIluBlock, 0, s >>>( v, b, x, gate );
+         ilu_trsv_kernel< Real, false ><<< grid, kIluBlock, 0, s >>>( v, b, x );
       ilu_begin_kernel< Gate ><<< 1, 1, 0, s >>>( v.st, gate );
       if( plain_sum )
-         ilu_trsv_kernel< Real, true, Gate, true ><<< grid, kIluBlock, 0, s >>>( v, x, x, gate );
+         ilu_trsv_kernel< Real, true, true ><<< grid, kIluBlock, 0, s >>>( v, x, x );
       else
-         ilu_trsv_kernel< Real, true, Gate ><<< grid, kIluBlock, 0, s >>>( v, x, x, gate );
+         ilu_trsv_kernel< Real, true ><<< grid, kIluBlock, 0, s >>>( v, x, x );
+      B2S_TRY_CUDA( cudaGetLastError() );
+      return B2S_OK;
+   }
+
+   template< bool PLAIN, class Gate >
+   b2s_status apply_blocks( const Real* b, Real* x, cudaStream_t s, Gate gate ) const
+   {
+      using Bits = typename TrsvBits< Real >::type;
+      Bits *y = yz.as< Bits >(), *z = y + n;
+      const size_t smem = (size_t) rows_per_block * sizeof( Real );
+      B2S_TRY( allow_smem( reinterpret_cast< const void* >( ilu_block_trsv_kernel< Real, false, PLAIN, Gate > ), smem ) );
+      B2S_TRY( allow_smem( reinterpret_cast< const void* >( ilu_block_trsv_kernel< Real, true, PLAIN, Gate > ), smem ) );
+      ilu_block_trsv_kernel< Real, false, PLAIN, Gate >
+         <<< blocks, kTrsvBlock, smem, s >>>( plan_l.view( n, rows_per_block ), state.as< IluState >(), b, y, z, x, gate );
+      ilu_block_trsv_kernel< Real, true, PLAIN, Gate ><<< blocks, kTrsvBlock, smem, s >>>(
+         plan_u.view( n, rows_per_block ), state.as< IluState >(), reinterpret_cast< const Real* >( y ), z, y, x, gate );
+      B2S_TRY_CUDA( cudaGetLastError() );
+      return B2S_OK;
+   }
+
+   // both scratch vectors to the pending value
+   b2s_status clear_scratch( cudaStream_t s ) const
+   {
+      using Bits = typename TrsvBits< Real >::type;
+      trsv_clear_kernel< Bits ><<< 256, 256, 0, s >>>( yz.as< Bits >(), 2 * (int64_t) n, TrsvBits< Real >::pending );
       B2S_TRY_CUDA( cudaGetLastError() );
       return B2S_OK;
    }
@@ -302,6 +679,8 @@ struct IluFactors
       if( h.error ) {
          const int zero = 0;
          B2S_TRY( copy_h2d( reinterpret_cast< char* >( state.p ) + offsetof( IluState, error ), &zero, sizeof( int ), s ) );
+         if( blocks > 0 )
+            B2S_TRY( clear_scratch( s ) );
          set_error( "ILU(0): a bounded wait for a dependency gave up" );
          return B2S_TIMEOUT;
       }
@@ -314,10 +693,15 @@ template< typename Real >
 b2s_status ilu_factorize( const b2s_matrix_t* A, const Real* values, IluFactors< Real >& F, cudaStream_t s );
 
 // The level orders of F's L and U dependency graphs from the host copy of its
-// pattern (hdiag: the first U position of each row), and the pass state.
+// pattern (hdiag: the first U position of each row), the pass state, and the
+// block plans where the rows suit them.
 template< typename Real >
 b2s_status ilu_levels( IluFactors< Real >& F, const std::vector< int32_t >& hoff, const std::vector< int32_t >& hcol,
                        const std::vector< int32_t >& hdiag, cudaStream_t s );
+
+// The block plans' slots from the computed factors.
+template< typename Real >
+b2s_status ilu_pack( IluFactors< Real >& F, cudaStream_t s );
 
 // ILUT( p, tau ) factors of A in the ILU(0) factor structure, applied by the
 // same kernels with PLAIN sums (ilut.cu).

@@ -242,6 +242,7 @@ ilut_factorize( const b2s_matrix_t* A, int32_t p, double tau_d, IluFactors< Real
    if( n == 0 )
       return B2S_OK;
    B2S_TRY( ilu_levels( F, foff, fcol, fdiag, s ) );
+   B2S_TRY( ilu_pack( F, s ) );
    B2S_TRY_CUDA( cudaStreamSynchronize( s ) );
    return B2S_OK;
 }
