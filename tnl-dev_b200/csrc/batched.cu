@@ -10,9 +10,14 @@
 // partials in rank order, so all of them take the same decisions and the
 // result does not depend on timing. Between the three phases of an iteration
 // the cluster synchronizes with barrier.cluster (no global memory flags, no
-// spin waits). With C SMs per system only 148/C systems are active at a
-// time, which keeps their matrices and Krylov vectors resident in the 126 MB
-// L2; C is chosen by the autotuner from timed samples of the batch.
+// spin waits). C is chosen by the autotuner from timed samples of the batch.
+//
+// What bounds it is L2 traffic: per row, right-hand side and iteration the
+// direction P is gathered once per nonzero and X, R and AP are read and
+// written. Where a CTA's rows of P fit its shared memory (and then R, then AP)
+// they stay there, P gathered from it and, at the edge of a CTA's rows, from
+// the other CTAs' (solve_system). 512 systems of 1k to 65k rows, 1 to 8
+// right-hand sides: 324 -> 188 ms; 60 systems of up to 10k rows: 13.2 -> 4.7 ms.
 //
 // Right-hand sides of one system are interleaved (element (i, j) at
 // i*k + j), so one pass over a matrix row serves all k of them.
@@ -26,6 +31,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <numeric>
 #include <vector>
@@ -37,6 +43,7 @@ namespace b2s {
 constexpr int kBatchBlock = 1024;
 constexpr int kBatchMaxRhs = 8;
 constexpr int kBatchWarps = kBatchBlock / 32;
+constexpr size_t kBatchSmem = 208 * 1024;  // per CTA (one CTA per SM), beside the static state
 
 struct BatchArgs
 {
@@ -59,6 +66,7 @@ struct BatchArgs
    unsigned int* counter;
    double tol, div_tol;
    int64_t maxit, minit;
+   int smem_elems;  // doubles of dynamic shared memory per CTA
    int64_t* t_sys;  // optional (autotuner): global-timer ns at start and end of each system
 };
 
@@ -74,55 +82,12 @@ global_ns()
 template< int K >
 struct SysState
 {
-   double part[ 2 ][ 2 * K ];  // this CTA's partial sums (double buffered)
-   double red[ kBatchWarps ][ 2 * K ];
+   double part[ 2 ][ K ];  // this CTA's partial sums (double buffered)
+   double red[ K ][ kBatchWarps ];
    double normb[ K ], s1[ K ], alpha[ K ], beta[ K ], residue[ K ];
    long long it[ K ];
    int done[ K ], reason[ K ];
 };
-
-// Sum of NR values over the CTA (fixed order); the CTA's total lands in
-// part[0..NR). `red` holds kBatchWarps rows of `ld` doubles.
-template< int NR >
-__device__ __forceinline__ void
-cta_partial( double ( &v )[ NR ], double* red, int ld, double* part )
-{
-   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-   for( int k = 0; k < NR; k++ ) {
-      double s = v[ k ];
-#pragma unroll
-      for( int o = 16; o > 0; o >>= 1 )
-         s += __shfl_xor_sync( 0xffffffffu, s, o );
-      if( lane == 0 )
-         red[ warp * ld + k ] = s;
-   }
-   __syncthreads();
-   if( threadIdx.x < NR ) {
-      double s = 0;
-      for( int w = 0; w < kBatchWarps; w++ )
-         s += red[ w * ld + threadIdx.x ];
-      part[ threadIdx.x ] = s;
-   }
-}
-
-// Cluster-wide totals of NR values: every CTA sums the C partials in rank order.
-template< int NR >
-__device__ __forceinline__ void
-cluster_total( cg::cluster_group& cl, double* part, double ( &tot )[ NR ] )
-{
-   cl.sync();
-   const int C = (int) cl.num_blocks();
-#pragma unroll
-   for( int k = 0; k < NR; k++ )
-      tot[ k ] = 0.0;
-   for( int q = 0; q < C; q++ ) {
-      const double* pq = cl.map_shared_rank( part, q );
-#pragma unroll
-      for( int k = 0; k < NR; k++ )
-         tot[ k ] += pq[ k ];
-   }
-}
 
 // IterativeSolver::checkNextIteration / nextIteration for one right-hand side
 __device__ __forceinline__ void
@@ -137,14 +102,48 @@ next_iteration_rhs( double residue, long long& it, int& done, int& reason, const
    }
 }
 
-// y(rows) = A p over the CTA's rows of the system, K columns at once;
-// `fn( i_local, acc )` receives each row's K sums.
+// Cluster-wide sums of K values in a fixed order: lanes, then warps (warp j
+// sums value j), then the C CTAs in rank order. Thread j < K hands the total
+// of value j to `fn( j, total )`, so the right-hand sides' scalar work runs
+// side by side; what it writes is visible to the CTA on return.
 template< int K, class F >
 __device__ __forceinline__ void
-spmm_rows( const BatchArgs& a, int64_t row0, int64_t r_begin, int64_t r_end, const double* p, F&& fn )
+cluster_sum( cg::cluster_group& cl, SysState< K >& st, int& buf, double ( &v )[ K ], F&& fn )
 {
-   for( int64_t i = r_begin + threadIdx.x; i < r_end; i += kBatchBlock ) {
-      const int64_t gr = row0 + i;
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+   for( int j = 0; j < K; j++ ) {
+      const double s = warp_sum( v[ j ] );
+      if( lane == 0 )
+         st.red[ j ][ warp ] = s;
+   }
+   __syncthreads();
+   if( warp < K ) {
+      const double s = warp_sum( lane < kBatchWarps ? st.red[ warp ][ lane ] : 0.0 );
+      if( lane == 0 )
+         st.part[ buf ][ warp ] = s;
+   }
+   cl.sync();
+   if( threadIdx.x < K ) {
+      const int j = threadIdx.x, C = (int) cl.num_blocks();
+      double t = 0.0;
+      for( int q = 0; q < C; q++ )
+         t += cl.map_shared_rank( &st.part[ buf ][ 0 ], q )[ j ];
+      fn( j, t );
+   }
+   __syncthreads();
+   buf ^= 1;
+}
+
+// y(rows) = A p over the CTA's rows of the system, K columns at once:
+// `gather( c, xs )` gives the K entries at column c (local to the system),
+// `fn( i, acc )` receives each row's K sums (i counted from r_begin).
+template< int K, class G, class F >
+__device__ __forceinline__ void
+spmm_rows( const BatchArgs& a, int64_t row0, int r_begin, int rows, G&& gather, F&& fn )
+{
+   for( int i = threadIdx.x; i < rows; i += kBatchBlock ) {
+      const int64_t gr = row0 + r_begin + i;
       const int b = __ldg( a.off + gr ), e = __ldg( a.off + gr + 1 );
       double acc[ K ];
 #pragma unroll
@@ -163,10 +162,11 @@ spmm_rows( const BatchArgs& a, int64_t row0, int64_t r_begin, int64_t r_end, con
 #pragma unroll
          for( int u = 0; u < 4; u++ ) {
             if( t0 + u < e ) {
-               const double* pc = p + (int64_t) lc[ u ] * K;
+               double xs[ K ];
+               gather( lc[ u ], xs );
 #pragma unroll
                for( int j = 0; j < K; j++ )
-                  acc[ j ] += v[ u ] * __ldcg( pc + j );  // written by other CTAs: read through L2
+                  acc[ j ] += v[ u ] * xs[ j ];
             }
          }
       }
@@ -174,21 +174,37 @@ spmm_rows( const BatchArgs& a, int64_t row0, int64_t r_begin, int64_t r_end, con
    }
 }
 
-template< int K >
+// One system on one cluster. PS: the direction P sits in the CTAs' shared
+// memory (`smem`, a.smem_elems doubles each), where the product gathers it
+// (other CTAs' rows through distributed shared memory), and R and AP too as
+// far as they fit; otherwise P goes through L2. The vectors are kept by
+// right-hand side (element (i, j) at j * ld + i), so a warp's accesses to one
+// right-hand side are consecutive in either memory; with PS, X is worked on
+// in that order too, in the buffer that P would take.
+template< int K, bool PS >
 __device__ void
-solve_system( const BatchArgs& a, int sys, cg::cluster_group& cl, SysState< K >& st )
+solve_system( const BatchArgs& a, int sys, cg::cluster_group& cl, SysState< K >& st, double* smem )
 {
    const int C = (int) cl.num_blocks(), q = (int) cl.block_rank();
-   const int64_t row0 = a.row_ptr[ sys ], n = a.row_ptr[ sys + 1 ] - row0;
-   const int64_t r_begin = n * q / C, r_end = n * ( q + 1 ) / C;
+   const int64_t row0 = a.row_ptr[ sys ];
+   const int n = (int) ( a.row_ptr[ sys + 1 ] - row0 );
+   const int per = ( n + C - 1 ) / C;  // rows per CTA
+   const int r_begin = min( n, q * per ), rows = min( n, r_begin + per ) - r_begin;
    const int64_t vo = a.vec_off[ sys ];
-   const double* B = a.B + vo;
+   const double* B = a.B + vo + (int64_t) r_begin * K;
    double* X = a.X + vo;
-   double* R = a.R + vo;
-   double* P = a.P + vo;
-   double* AP = a.AP + vo;
-   const double* dg = a.diag ? a.diag + row0 : nullptr;
+   const double* dg = a.diag ? a.diag + row0 + r_begin : nullptr;
    int buf = 0;
+   // where the vectors live: pointer to this CTA's first row, distance between right-hand sides
+   const int fit = PS ? a.smem_elems / max( 1, per * K ) : 0;  // vectors that fit (P, then R, then AP)
+   double *P, *R, *AP;
+   const int64_t ldP = PS ? per : n;
+   const int64_t ldR = fit >= 2 ? per : n, ldA = fit >= 3 ? per : n;
+   P = PS ? smem : a.P + vo + r_begin;
+   R = fit >= 2 ? smem + per * K : a.R + vo + r_begin;
+   AP = fit >= 3 ? smem + 2 * per * K : a.AP + vo + r_begin;
+   double* xw = PS ? a.P + vo + r_begin : X + (int64_t) r_begin * K;
+   const int xi = PS ? 1 : K, xj = PS ? n : 1;
 
    // ||M^-1 b|| per right-hand side (CG.hpp:24-32)
    {
@@ -196,24 +212,17 @@ solve_system( const BatchArgs& a, int sys, cg::cluster_group& cl, SysState< K >&
 #pragma unroll
       for( int j = 0; j < K; j++ )
          v[ j ] = 0.0;
-      for( int64_t i = r_begin + threadIdx.x; i < r_end; i += kBatchBlock ) {
+      for( int i = threadIdx.x; i < rows; i += kBatchBlock ) {
          const double d = dg ? dg[ i ] : 1.0;
 #pragma unroll
          for( int j = 0; j < K; j++ ) {
-            const double t = dg ? B[ i * K + j ] / d : B[ i * K + j ];
+            const double t = dg ? B[ (int64_t) i * K + j ] / d : B[ (int64_t) i * K + j ];
             v[ j ] += t * t;
          }
       }
-      cta_partial< K >( v, &st.red[ 0 ][ 0 ], 2 * K, st.part[ buf ] );
-      double tot[ K ];
-      cluster_total< K >( cl, st.part[ buf ], tot );
-      buf ^= 1;
-      if( threadIdx.x == 0 )
-         for( int j = 0; j < K; j++ ) {
-            st.normb[ j ] = sqrt( tot[ j ] );
-            if( st.normb[ j ] == 0.0 )
-               st.normb[ j ] = 1.0;
-         }
+      cluster_sum< K >( cl, st, buf, v, [ & ]( int j, double t ) {
+         st.normb[ j ] = t == 0.0 ? 1.0 : sqrt( t );
+      } );
    }
    // r = b - A x ; z = M^-1 r ; p = z ; s1 = (r, z) (CG.hpp:37-58)
    {
@@ -221,31 +230,34 @@ solve_system( const BatchArgs& a, int sys, cg::cluster_group& cl, SysState< K >&
 #pragma unroll
       for( int j = 0; j < K; j++ )
          v[ j ] = 0.0;
-      spmm_rows< K >( a, row0, r_begin, r_end, X, [ & ]( int64_t i, const double( &acc )[ K ] ) {
-         const double d = dg ? dg[ i ] : 1.0;
+      spmm_rows< K >(
+         a, row0, r_begin, rows,
+         [ & ]( int c, double( &xs )[ K ] ) {
 #pragma unroll
-         for( int j = 0; j < K; j++ ) {
-            const double r = B[ i * K + j ] - acc[ j ];
-            const double z = dg ? r / d : r;
-            R[ i * K + j ] = r;
-            P[ i * K + j ] = z;
-            v[ j ] += r * z;
-         }
+            for( int j = 0; j < K; j++ )
+               xs[ j ] = X[ (int64_t) c * K + j ];
+         },
+         [ & ]( int i, const double( &acc )[ K ] ) {
+            const double d = dg ? dg[ i ] : 1.0;
+#pragma unroll
+            for( int j = 0; j < K; j++ ) {
+               const double r = B[ (int64_t) i * K + j ] - acc[ j ];
+               const double z = dg ? r / d : r;
+               R[ j * ldR + i ] = r;
+               P[ j * ldP + i ] = z;
+               if( PS )
+                  xw[ j * xj + i ] = X[ (int64_t) ( r_begin + i ) * K + j ];
+               v[ j ] += r * z;
+            }
+         } );
+      cluster_sum< K >( cl, st, buf, v, [ & ]( int j, double t ) {
+         st.s1[ j ] = t;
+         st.it[ j ] = 0;
+         st.done[ j ] = 0;
+         st.reason[ j ] = 0;
+         st.residue[ j ] = sqrt( t ) / st.normb[ j ];
+         next_iteration_rhs( st.residue[ j ], st.it[ j ], st.done[ j ], st.reason[ j ], a );
       } );
-      cta_partial< K >( v, &st.red[ 0 ][ 0 ], 2 * K, st.part[ buf ] );
-      double tot[ K ];
-      cluster_total< K >( cl, st.part[ buf ], tot );
-      buf ^= 1;
-      if( threadIdx.x == 0 )
-         for( int j = 0; j < K; j++ ) {
-            st.s1[ j ] = tot[ j ];
-            st.it[ j ] = 0;
-            st.done[ j ] = 0;
-            st.reason[ j ] = 0;
-            st.residue[ j ] = sqrt( tot[ j ] ) / st.normb[ j ];
-            next_iteration_rhs( st.residue[ j ], st.it[ j ], st.done[ j ], st.reason[ j ], a );
-         }
-      __syncthreads();
    }
    for( ;; ) {
       bool any = false;
@@ -262,32 +274,51 @@ solve_system( const BatchArgs& a, int sys, cg::cluster_group& cl, SysState< K >&
 #pragma unroll
          for( int j = 0; j < K; j++ )
             v[ j ] = 0.0;
-         spmm_rows< K >( a, row0, r_begin, r_end, P, [ & ]( int64_t i, const double( &acc )[ K ] ) {
+         spmm_rows< K >(
+            a, row0, r_begin, rows,
+            [ & ]( int c, double( &xs )[ K ] ) {
+               const double* p;
+               if constexpr( PS ) {
+                  const int i = c - r_begin;
+                  if( i >= 0 && i < rows ) {
 #pragma unroll
-            for( int j = 0; j < K; j++ ) {
-               AP[ i * K + j ] = acc[ j ];
-               v[ j ] += acc[ j ] * P[ i * K + j ];
-            }
-         } );
-         cta_partial< K >( v, &st.red[ 0 ][ 0 ], 2 * K, st.part[ buf ] );
-         double tot[ K ];
-         cluster_total< K >( cl, st.part[ buf ], tot );
-         buf ^= 1;
-         if( threadIdx.x == 0 )
-            for( int j = 0; j < K; j++ ) {
-               if( st.done[ j ] )
-                  continue;
-               if( tot[ j ] == 0.0 ) {
-                  // p = 0 => r = 0: solved (CG.hpp:64-67)
-                  st.residue[ j ] = 0.0;
-                  st.done[ j ] = 1;
-                  st.reason[ j ] = 2;
-                  st.alpha[ j ] = 0.0;
+                     for( int j = 0; j < K; j++ )
+                        xs[ j ] = smem[ j * per + i ];
+                     return;
+                  }
+                  const int owner = c / per;
+                  p = cl.map_shared_rank( smem, owner ) + ( c - owner * per );
+#pragma unroll
+                  for( int j = 0; j < K; j++ )
+                     xs[ j ] = p[ j * per ];
                }
-               else
-                  st.alpha[ j ] = st.s1[ j ] / tot[ j ];
+               else {
+                  p = a.P + vo + c;
+#pragma unroll
+                  for( int j = 0; j < K; j++ )
+                     xs[ j ] = __ldcg( p + (int64_t) j * n );  // written by other CTAs: read through L2
+               }
+            },
+            [ & ]( int i, const double( &acc )[ K ] ) {
+#pragma unroll
+               for( int j = 0; j < K; j++ ) {
+                  AP[ j * ldA + i ] = acc[ j ];
+                  v[ j ] += acc[ j ] * P[ j * ldP + i ];
+               }
+            } );
+         cluster_sum< K >( cl, st, buf, v, [ & ]( int j, double t ) {
+            if( st.done[ j ] )
+               return;
+            if( t == 0.0 ) {
+               // p = 0 => r = 0: solved (CG.hpp:64-67)
+               st.residue[ j ] = 0.0;
+               st.done[ j ] = 1;
+               st.reason[ j ] = 2;
+               st.alpha[ j ] = 0.0;
             }
-         __syncthreads();
+            else
+               st.alpha[ j ] = st.s1[ j ] / t;
+         } );
       }
       // x += alpha p ; r -= alpha Ap ; z = M^-1 r ; s1 = (r, z)
       {
@@ -299,34 +330,28 @@ solve_system( const BatchArgs& a, int sys, cg::cluster_group& cl, SysState< K >&
             act[ j ] = ! st.done[ j ];
             v[ j ] = 0.0;
          }
-         for( int64_t i = r_begin + threadIdx.x; i < r_end; i += kBatchBlock ) {
+         for( int i = threadIdx.x; i < rows; i += kBatchBlock ) {
             const double d = dg ? dg[ i ] : 1.0;
 #pragma unroll
             for( int j = 0; j < K; j++ ) {
                if( ! act[ j ] )
                   continue;
-               const int64_t e = i * K + j;
-               X[ e ] += al[ j ] * P[ e ];
-               const double r = R[ e ] - al[ j ] * AP[ e ];
-               R[ e ] = r;
+               double* x = xw + (int64_t) i * xi + (int64_t) j * xj;
+               *x += al[ j ] * P[ j * ldP + i ];
+               const double r = R[ j * ldR + i ] - al[ j ] * AP[ j * ldA + i ];
+               R[ j * ldR + i ] = r;
                v[ j ] += dg ? r * ( r / d ) : r * r;
             }
          }
-         cta_partial< K >( v, &st.red[ 0 ][ 0 ], 2 * K, st.part[ buf ] );
-         double tot[ K ];
-         cluster_total< K >( cl, st.part[ buf ], tot );
-         buf ^= 1;
-         if( threadIdx.x == 0 )
-            for( int j = 0; j < K; j++ ) {
-               if( st.done[ j ] )
-                  continue;
-               const double s2 = st.s1[ j ];
-               st.s1[ j ] = tot[ j ];
-               st.beta[ j ] = s2 == 0.0 ? 0.0 : tot[ j ] / s2;
-               st.residue[ j ] = sqrt( tot[ j ] ) / st.normb[ j ];
-               next_iteration_rhs( st.residue[ j ], st.it[ j ], st.done[ j ], st.reason[ j ], a );
-            }
-         __syncthreads();
+         cluster_sum< K >( cl, st, buf, v, [ & ]( int j, double t ) {
+            if( st.done[ j ] )
+               return;
+            const double s2 = st.s1[ j ];
+            st.s1[ j ] = t;
+            st.beta[ j ] = s2 == 0.0 ? 0.0 : t / s2;
+            st.residue[ j ] = sqrt( t ) / st.normb[ j ];
+            next_iteration_rhs( st.residue[ j ], st.it[ j ], st.done[ j ], st.reason[ j ], a );
+         } );
       }
       // p = z + beta p
       {
@@ -337,19 +362,23 @@ solve_system( const BatchArgs& a, int sys, cg::cluster_group& cl, SysState< K >&
             be[ j ] = st.beta[ j ];
             act[ j ] = ! st.done[ j ];
          }
-         for( int64_t i = r_begin + threadIdx.x; i < r_end; i += kBatchBlock ) {
+         for( int i = threadIdx.x; i < rows; i += kBatchBlock ) {
             const double d = dg ? dg[ i ] : 1.0;
 #pragma unroll
             for( int j = 0; j < K; j++ ) {
                if( ! act[ j ] )
                   continue;
-               const int64_t e = i * K + j;
-               const double z = dg ? R[ e ] / d : R[ e ];
-               P[ e ] = z + be[ j ] * P[ e ];
+               const double r = R[ j * ldR + i ];
+               P[ j * ldP + i ] = ( dg ? r / d : r ) + be[ j ] * P[ j * ldP + i ];
             }
          }
       }
    }
+   if( PS )
+      for( int i = threadIdx.x; i < rows; i += kBatchBlock )
+#pragma unroll
+         for( int j = 0; j < K; j++ )
+            X[ (int64_t) ( r_begin + i ) * K + j ] = xw[ j * xj + i ];
    // report (rank 0)
    if( q == 0 && threadIdx.x < K ) {
       const int j = threadIdx.x;
@@ -374,6 +403,7 @@ batch_cg_kernel( BatchArgs a )
    cg::cluster_group cl = cg::this_cluster();
    __shared__ __align__( 16 ) unsigned char smem_raw[ sizeof( SysState< kBatchMaxRhs > ) ];
    __shared__ int next_sys;
+   extern __shared__ __align__( 16 ) double batch_smem[];
    for( ;; ) {
       if( cl.block_rank() == 0 && threadIdx.x == 0 )
          next_sys = (int) atomicAdd( a.counter, 1u );
@@ -387,10 +417,16 @@ batch_cg_kernel( BatchArgs a )
       const bool stamp = a.t_sys && cl.block_rank() == 0 && threadIdx.x == 0;
       if( stamp )
          a.t_sys[ 2 * sys ] = global_ns();
+      // the direction of the largest CTA's rows in shared memory
+      const int64_t C = cl.num_blocks(), rows = a.row_ptr[ sys + 1 ] - a.row_ptr[ sys ];
+      const bool in_smem = ( rows + C - 1 ) / C * a.nrhs[ sys ] <= a.smem_elems;
       switch( a.nrhs[ sys ] ) {
 #define B2S_BATCH_K( KK )                                                                            \
    case KK:                                                                                          \
-      solve_system< KK >( a, sys, cl, *reinterpret_cast< SysState< KK >* >( smem_raw ) );          \
+      if( in_smem )                                                                                  \
+         solve_system< KK, true >( a, sys, cl, *reinterpret_cast< SysState< KK >* >( smem_raw ), batch_smem );  \
+      else                                                                                           \
+         solve_system< KK, false >( a, sys, cl, *reinterpret_cast< SysState< KK >* >( smem_raw ), batch_smem ); \
       break;
          B2S_BATCH_K( 1 )
          B2S_BATCH_K( 2 )
@@ -472,6 +508,7 @@ launch_batch( b2s_batch_t* bt, const double* B, double* X, int cluster, int nsys
    a.div_tol = bt->o.divergence_residue;
    a.maxit = maxit;
    a.minit = bt->o.min_iterations;
+   a.smem_elems = (int) ( kBatchSmem / sizeof( double ) );
    a.t_sys = t_sys;
    B2S_TRY_CUDA( cudaMemsetAsync( bt->counter.p, 0, sizeof( unsigned int ), s ) );
    cudaLaunchConfig_t cfg{};
@@ -481,7 +518,8 @@ launch_batch( b2s_batch_t* bt, const double* B, double* X, int cluster, int nsys
    attr[ 0 ].val.clusterDim.y = 1;
    attr[ 0 ].val.clusterDim.z = 1;
    cfg.blockDim = dim3( kBatchBlock );
-   cfg.dynamicSmemBytes = 0;
+   cfg.dynamicSmemBytes = kBatchSmem;
+   B2S_TRY( allow_smem( reinterpret_cast< const void* >( batch_cg_kernel ), kBatchSmem ) );
    cfg.stream = s;
    cfg.attrs = attr;
    cfg.numAttrs = 1;
@@ -501,21 +539,23 @@ launch_batch( b2s_batch_t* bt, const double* B, double* X, int cluster, int nsys
 }
 
 // Autotuner of the cluster size. A sample of systems (even strides through
-// the size-sorted queue) is solved to convergence under every candidate C
-// while the kernel stamps each system's start and end. For C the full batch
-// is predicted as
-//     max( sum over the batch of (duration x C) / (resident clusters x C),
-//          longest single system )
-// — the SM time the systems need spread over the device, or the tail of the
-// slowest one, whichever is longer — scaling the sample's SM time by
-// nsys / sample. The C with the smallest prediction wins.
+// the size-sorted queue) is solved from X under every candidate C while the
+// kernel stamps each system's start and end: to convergence under the first C,
+// which tells the systems' iterations, under the others for kTuneIterations,
+// scaled to them. Every system of the queue is then taken to last as long as
+// its neighbour in the sample, and the queue is played through on the resident
+// clusters of C; the C whose last system ends first wins. (The systems' total
+// time spread over the device, or the longest of them, leaves out the tail
+// where a few long systems run alone.)
+// W: the sample's solutions.
+constexpr int64_t kTuneIterations = 32;
+
 static b2s_status
-autotune_cluster( b2s_batch_t* bt, const double* B, double* X, cudaStream_t s, int& best )
+autotune_cluster( b2s_batch_t* bt, const double* B, const double* X, double* W, cudaStream_t s, int& best )
 {
    best = 1;
-   const int cands[] = { 1, 2, 4, 8 };
-   const int sms = num_sms();
-   const int sample = std::min( bt->nsys, 2 * sms );
+   const int cands[] = { 8, 4, 2, 1 };
+   const int sample = std::min( bt->nsys, 2 * num_sms() );
    std::vector< int32_t > order_h( bt->nsys );
    B2S_TRY( copy_d2h( order_h.data(), bt->order.p, bt->nsys * sizeof( int32_t ), s ) );
    std::vector< int32_t > pick( sample );
@@ -525,27 +565,39 @@ autotune_cluster( b2s_batch_t* bt, const double* B, double* X, cudaStream_t s, i
    B2S_TRY( sample_order.alloc( sample * sizeof( int32_t ) ) );
    B2S_TRY( copy_h2d( sample_order.p, pick.data(), sample * sizeof( int32_t ), s ) );
    B2S_TRY( stamps.alloc( (size_t) 2 * bt->nsys * sizeof( int64_t ) ) );
-   std::vector< int64_t > t( 2 * bt->nsys );
+   std::vector< int64_t > t( 2 * bt->nsys ), its( bt->nslots );
+   std::vector< double > scale;  // a system's iterations over the timed ones
    double best_est = 1e300;
    for( int c : cands ) {
       int nclusters = 0;
-      b2s_status st = launch_batch( bt, B, X, c, sample, bt->o.max_iterations, s, sample_order.as< int32_t >(),
-                                    stamps.as< int64_t >(), &nclusters );
+      B2S_TRY_CUDA( cudaMemcpyAsync( W, X, bt->nvec * sizeof( double ), cudaMemcpyDeviceToDevice, s ) );
+      const bool all = scale.empty();
+      const b2s_status st = launch_batch( bt, B, W, c, sample, all ? bt->o.max_iterations : std::min< int64_t >( bt->o.max_iterations, kTuneIterations ), s,
+                                          sample_order.as< int32_t >(), stamps.as< int64_t >(), &nclusters );
       if( st != B2S_OK ) {
          cudaGetLastError();
          clear_error();
          continue;
       }
       B2S_TRY( copy_d2h( t.data(), stamps.p, t.size() * sizeof( int64_t ), s ) );
-      double sm_ns = 0, longest = 0;
-      for( int k = 0; k < sample; k++ ) {
-         const int sys = pick[ k ];
-         const double d = (double) ( t[ 2 * sys + 1 ] - t[ 2 * sys ] );
-         sm_ns += d * c;
-         longest = std::max( longest, d );
+      if( all ) {
+         B2S_TRY( copy_d2h( its.data(), bt->it_out.p, bt->nslots * sizeof( int64_t ), s ) );
+         for( const int sys : pick ) {
+            int64_t most = 1;
+            for( int j = 0; j < bt->nrhs_h[ sys ]; j++ )
+               most = std::max( most, its[ bt->rhs_off_h[ sys ] + j ] );
+            scale.push_back( std::max( 1.0, (double) most / (double) ( kTuneIterations + 1 ) ) );
+         }
       }
-      const double total_sm_ns = sm_ns * ( (double) bt->nsys / sample );
-      const double est = std::max( total_sm_ns / ( (double) std::max( nclusters, 1 ) * c ), longest );
+      std::vector< double > ends( (size_t) std::max( nclusters, 1 ), 0.0 );  // a heap, the earliest first
+      double est = 0;
+      for( int k = 0; k < bt->nsys; k++ ) {
+         const int q = (int) ( (int64_t) k * sample / bt->nsys ), sys = pick[ q ];
+         std::pop_heap( ends.begin(), ends.end(), std::greater< double >() );
+         ends.back() += (double) ( t[ 2 * sys + 1 ] - t[ 2 * sys ] ) * ( all ? 1.0 : scale[ q ] );
+         est = std::max( est, ends.back() );
+         std::push_heap( ends.begin(), ends.end(), std::greater< double >() );
+      }
       if( est < best_est ) {
          best_est = est;
          best = c;
@@ -690,12 +742,11 @@ b2s_batch_solve( b2s_batch bt, const double* B, double* X, b2s_stream stream, b2
       return B2S_OK;
    }
    if( bt->cluster == 0 ) {
-      // autotune on a copy of the initial guess so X is untouched
+      // autotune on copies of the initial guess so X is untouched
       DevBuf xs;
       B2S_TRY( xs.alloc( bt->nvec * sizeof( double ) ) );
-      B2S_TRY_CUDA( cudaMemcpyAsync( xs.p, X, bt->nvec * sizeof( double ), cudaMemcpyDeviceToDevice, s ) );
       int best = 1;
-      B2S_TRY( autotune_cluster( bt, B, xs.as< double >(), s, best ) );
+      B2S_TRY( autotune_cluster( bt, B, X, xs.as< double >(), s, best ) );
       B2S_TRY_CUDA( cudaStreamSynchronize( s ) );
       bt->cluster = best;
    }
