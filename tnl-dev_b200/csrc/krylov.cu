@@ -15,6 +15,7 @@
 #include "krylov_kernels.cuh"
 #include "tfqmr_bicgstabl.cuh"
 #include "ilu.cuh"
+#include "resident.cuh"
 #include "stationary.cuh"
 
 #include <algorithm>
@@ -815,6 +816,10 @@ struct b2s_solver_t
    // FP64 outer vectors (mixed)
    DevBuf outer;
 
+   // exchange slots of the resident CG / BiCGStab kernel (empty: the graph of
+   // kernels runs)
+   DevBuf resident;
+
    // GMRES
    DevBuf gm;
    DevBuf V;
@@ -1053,6 +1058,33 @@ normb_launch( b2s_solver_t* S, const Real* b, const Real* diag )
    return B2S_OK;
 }
 
+// Iterations of the resident kernel until it says done or stops early: it
+// runs at most `kResidentIterations` per launch, so that other streams get
+// their turn and the wall clock is looked at.
+constexpr int kResidentIterations = 1000;
+
+template< typename Real >
+static b2s_status
+resident_run( b2s_solver_t* S, const Real* vals, const Real* diag, double eps2 )
+{
+   auto v = vec_layout< Real >( S );
+   Ctl* ctl = S->ctl_buf.as< Ctl >();
+   const ResidentVecs< Real > rv{ v.x, v.r, v.p, v.Ap, v.z, v.r_ast, v.s, v.As };
+   const int iterations = S->o.check_interval > 0 ? S->o.check_interval : kResidentIterations;
+   for( ;; ) {
+      B2S_TRY( resident_iterate< Real >( S->A, S->o.solver, vals, diag, rv, ctl, S->resident, iterations, eps2, S->cs ) );
+      B2S_TRY( read_ctl( S ) );
+      if( S->h_ctl->gave_up ) {
+         B2S_TRY( resident_scratch_init( S->resident, S->cs ) );
+         set_error( "solver: a bounded wait between blocks gave up" );
+         return B2S_TIMEOUT;
+      }
+      if( S->h_ctl->done || S->h_ctl->restart_flag )
+         return B2S_OK;
+      B2S_TRY( check_wall( S ) );
+   }
+}
+
 template< typename Real >
 static b2s_status cg_iterate( b2s_solver_t* S, const Real* vals, const Real* diag, long long tagbase );
 
@@ -1098,6 +1130,8 @@ cg_iterate( b2s_solver_t* S, const Real* vals, const Real* diag, long long tagba
    auto v = vec_layout< Real >( S );
    Ctl* ctl = S->ctl_buf.as< Ctl >();
    const IluFactors< Real >* ilu = ilu_of< Real >( S );
+   if( S->resident.p )
+      return resident_run< Real >( S, vals, diag, 0.0 );
    const int chunk = chunk_of( S );
    for( ;; ) {
       B2S_TRY( run_graph( S, tagbase + chunk, [ & ]() -> b2s_status
@@ -1199,6 +1233,17 @@ bicgstab_iterate( b2s_solver_t* S, const Real* vals, const Real* diag, long long
       s.exact = exact;
       return s;
    };
+   while( S->resident.p ) {
+      B2S_TRY( resident_run< Real >( S, vals, diag, eps * eps ) );
+      if( S->h_ctl->done )
+         return B2S_OK;
+      // r became too orthogonal to r_ast: a new r0, the next direction, and on
+      B2S_TRY( ( spmv_dispatch< Real, BiResG< Real > >( A, vals, v.x, 0, A->rows, res_sink( 1, v.r ), S->scr.slot( 6 ),
+                                                         S->cs ) ) );
+      vec_kernel< Real, BiPOp< Real >, NoFin ><<< wave_grid( vec_kernel< Real, BiPOp< Real >, NoFin >, n ), kReduceBlock, 0, S->cs >>>(
+         n, ctl, BiPOp< Real >{ v.p, v.r, v.Ap, Real( 0 ), Real( 0 ) }, NoFin{}, S->scr.slot( 8 ) );
+      B2S_TRY_CUDA( cudaGetLastError() );
+   }
    const int chunk = chunk_of( S );
    for( ;; ) {
       B2S_TRY( run_graph( S, tagbase + chunk, [ & ]() -> b2s_status
@@ -2135,7 +2180,7 @@ true_residual( b2s_solver_t* S, const Real* vals, const Real* b, const Real* x, 
    double* d_out = &S->ctl_buf.as< Ctl >()->outer_norm;  // reuse two doubles of the control block
    TrueResSink< Real > sink{ b, d_out };
    B2S_TRY( ( spmv_dispatch< Real, TrueResSink< Real > >( S->A, vals, x, 0, S->A->rows, sink, S->scr.slot( 9 ), S->cs ) ) );
-   double h[ 2 ];
+   double* h = &S->h_ctl->outer_norm;  // the host mirror is page-locked
    B2S_TRY_CUDA( cudaMemcpyAsync( h, d_out, 2 * sizeof( double ), cudaMemcpyDeviceToHost, S->cs ) );
    B2S_TRY_CUDA( cudaStreamSynchronize( S->cs ) );
    res = h[ 1 ] > 0 ? h[ 0 ] / h[ 1 ] : h[ 0 ];
@@ -2664,6 +2709,9 @@ b2s_solver_create( b2s_matrix A, const b2s_solve_opts* opts, b2s_solver* out )
       else
          B2S_TRY( ilut_factorize< float >( A, o.ilut_p, o.ilut_threshold, S->ilu32, S->cs ) );
    }
+   if( ( o.solver == B2S_CG || ( o.solver == B2S_BICGSTAB && ! o.bicgstab_exact_residue ) )
+       && o.preconditioner != B2S_PRECOND_ILU0 && o.preconditioner != B2S_PRECOND_ILUT && resident_fits( A, o.solver, es ) )
+      B2S_TRY( resident_scratch_init( S->resident, S->cs ) );
    if( o.solver == B2S_GMRES ) {
       const int M = o.gmres_restarting_max;
       S->mmax = M;

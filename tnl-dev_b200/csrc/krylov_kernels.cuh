@@ -21,6 +21,7 @@ struct Ctl
    long long it, maxit, minit;
    int done;       // no more work in this solve
    int reason;     // 0 running, 1 converged/stopped by check, 2 zero curvature, 3 breakdown
+   int gave_up;    // a bounded wait between the resident kernel's blocks ran out
    // shared scalars
    double normb;
    // CG
