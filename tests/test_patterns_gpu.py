@@ -1,8 +1,7 @@
 """Products through row patterns (one byte per row in place of the columns)
 against the oracle, at the limits of what is kept as patterns: 255 and 256
-patterns, rows of 64 and 65 elements, 2,048 offsets and more, empty rows,
-explicit zeros, rectangular matrices, counts around the warp, row-group and
-slice sizes; every layout that reads patterns, row ranges, both value types;
+patterns, rows of 64 and 65 elements, 2,040 and 2,400 offsets, empty rows, explicit zeros,
+rectangular matrices, the smallest matrix that has patterns and odd row counts; every layout that reads patterns, row ranges, both value types;
 and after the columns were permuted in place.
 
 Each row within the forward error bound of its dot product,
@@ -16,39 +15,51 @@ LAYOUTS = [("CSR", 0), ("Ellpack", 0), ("SlicedEllpack", 8), ("SlicedEllpack", 3
            ("ChunkedEllpack", 0), ("BiEllpack", 0)]
 
 
-def _rows(cols_of, cols, seed=0, zeros=False):
+N = 100000  # matrices below keep their columns
+
+
+def _rows(length, offsets_of, cols, seed=0, zeros=False, rows=N):
+    """Row i: the first length[i % len(length)] of offsets_of(i, k) + i inside [0, cols)."""
     g = np.random.default_rng(seed)
-    off = np.concatenate([[0], np.cumsum([len(c) for c in cols_of])]).astype(np.int32)
-    col = np.concatenate([np.asarray(c, np.int32) for c in cols_of] + [np.zeros(0, np.int32)])
+    i = np.arange(rows)
+    width = int(np.max(length)) if np.size(length) else 0
+    L = np.resize(np.asarray(length), rows)
+    c = i[:, None] + offsets_of(i[:, None], np.arange(width)[None, :]) if width else np.zeros((rows, 0), np.int64)
+    keep = (np.arange(width)[None, :] < L[:, None]) & (c >= 0) & (c < cols)
+    off = np.concatenate([[0], np.cumsum(keep.sum(axis=1))]).astype(np.int32)
+    col = c[keep].astype(np.int32)
     val = g.normal(size=len(col))
     if zeros and len(val):
-        val[g.integers(0, len(val), max(1, len(val) // 9))] = 0.0
-    return off, col.astype(np.int32), val, cols
+        val[g.integers(0, len(val), len(val) // 9)] = 0.0
+    return off, col, val, cols
 
 
 def _stencil(n, offsets, cols=None, **kw):
-    cols = n if cols is None else cols
-    return _rows([[i + o for o in offsets if 0 <= i + o < cols] for i in range(n)], cols, **kw)
+    o = np.asarray(offsets, np.int64)
+    return _rows([len(o)], lambda i, k: o[k] + 0 * i, n if cols is None else cols, rows=n, **kw)
 
 
-def _distinct(n, patterns, seed=1):
-    """`patterns` distinct rows {0, 1 + k}, the rest of the rows repeating them."""
-    return _rows([[i, i + 1 + i % patterns] for i in range(n)], n + patterns + 2, seed)
+def _distinct(patterns):
+    """`patterns` distinct rows {0, 1 + i % patterns}."""
+    return _rows([2], lambda i, k: np.where(k == 0, 0, 1 + i % patterns), N + patterns + 2)
 
 
 CASES = {
     "one_row": lambda: _stencil(1, [0]),
     "tri_31": lambda: _stencil(31, [-1, 0, 1]),
-    "five_4097": lambda: _stencil(4097, [-64, -1, 0, 1, 64]),
-    "seven_33x": lambda: _stencil(33 * 67, [-67, -33, -1, 0, 1, 33, 67], seed=3, zeros=True),
-    "wide": lambda: _stencil(700, [0, 3, 900], cols=1700),
-    "tall": lambda: _stencil(1700, [-900, -3, 0], cols=700),
-    "empty_rows": lambda: _rows([[] if i % 3 == 0 else [i // 3, 500 + i // 3] for i in range(1025)], 1100),
-    "patterns_255": lambda: _distinct(2000, 255),
-    "patterns_256": lambda: _distinct(2000, 256),
-    "row_64": lambda: _rows([list(range(i, i + (64 if i % 40 == 0 else 2))) for i in range(640)], 800),
-    "row_65": lambda: _rows([list(range(i, i + (65 if i % 40 == 0 else 2))) for i in range(640)], 800),
-    "offsets_over": lambda: _rows([list(range(i, i + 1 + i % 66)) for i in range(1980)], 2100),
+    "five_below": lambda: _stencil(N - 1, [-300, -1, 0, 1, 300]),
+    "five": lambda: _stencil(N, [-300, -1, 0, 1, 300]),
+    "five_odd": lambda: _stencil(N + 33, [-300, -1, 0, 1, 300], seed=2),
+    "seven_zeros": lambda: _stencil(N + 31, [-2500, -50, -1, 0, 1, 50, 2500], seed=3, zeros=True),
+    "wide": lambda: _stencil(N, [0, 3, 90000], cols=N + 70000),
+    "tall": lambda: _stencil(N + 1, [-90000, -3, 0], cols=N // 2),
+    "empty_rows": lambda: _rows([0, 2, 2], lambda i, k: 500 * k, N + 600),
+    "patterns_255": lambda: _distinct(255),
+    "patterns_256": lambda: _distinct(256),
+    "row_64": lambda: _rows([64] + [2] * 39, lambda i, k: k + 0 * i, N + 100),
+    "row_65": lambda: _rows([65] + [2] * 39, lambda i, k: k + 0 * i, N + 100),
+    "offsets_2040": lambda: _rows([60], lambda i, k: k + 2 * (i % 34), N + 200),
+    "offsets_2400": lambda: _rows([60], lambda i, k: k + 2 * (i % 40), N + 200),
 }
 
 
@@ -88,7 +99,7 @@ def test_pattern_products(b2s_lib, cuda, oracle, name, real):
 
 @pytest.mark.parametrize("segments", ["CSR", "SlicedEllpack", "BiEllpack"])
 def test_columns_permuted_in_place(b2s_lib, cuda, oracle, segments):
-    n = 900
+    n = N
     off, col, val, cols = _stencil(n, [-30, -1, 0, 1, 30])
     for iperm in (np.arange(n)[::-1].copy(), np.random.default_rng(2).permutation(n), np.roll(np.arange(n), 5)):
         iperm = iperm.astype(np.int32)

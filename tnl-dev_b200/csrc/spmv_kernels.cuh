@@ -584,19 +584,24 @@ load_patterns( const RowPatterns& P, PatternSmem& S )
 // row-group kernels issue instructions most of the time (0.6-0.7 per cycle and
 // scheduler), so this one counts them: 32-bit row arithmetic, eight elements at
 // a time under predicates.
-// Groups of values in flight or being summed per warp: three in FP32, whose
-// groups carry half the bytes (128^3 / 160^3 Laplacian 24.7 / 41.4 us against
-// 28.5 / 49.6 us with two), two in FP64 (33.1 against 34.3 us with three).
-template< typename Real >
-constexpr int kCsrPatStages = sizeof( Real ) == 4 ? 3 : 2;
+// kCsrPatStages groups of values are in flight or being summed per warp, and a
+// warp takes groups of 64 rows, lane l rows l and l + 32, which share the
+// group's staging. 128^3 / 160^3 Laplacian, us:
+//   FP32  32 rows, 2 stages 28.5 / 49.6; 3 stages 24.9 / 42.6
+//         64 rows, 2 stages 22.7 / 39.1; 3 stages 23.6 / 40.6
+//   FP64  32 rows, 2 stages 31.7 / 57.4; 3 stages 34.7 / 61.2
+//         64 rows, 2 stages 31.2 / 55.5
+constexpr int kCsrPatStages = 2;
+constexpr int kCsrPatRows = 2;  // rows per lane
 template< typename Real, class Sink >
-__global__ void __launch_bounds__( kCsrGroupBlock, 8 )
+__global__ void __launch_bounds__( kCsrGroupBlock, sizeof( Real ) == 4 ? 8 : 4 )
 csr_pattern_kernel( const int32_t* __restrict__ off, RowPatterns P, const Real* __restrict__ val,
                     const Real* __restrict__ x, int32_t row_begin, int32_t row_end, Sink sink, RedScratch rs )
 {
    constexpr int VPC = 16 / sizeof( Real );  // values per 16-byte chunk
-   constexpr int SC = kCsrGroupCap + 8;      // room for the alignment slack
-   constexpr int NS = kCsrPatStages< Real >;
+   constexpr int RPL = kCsrPatRows;
+   constexpr int SC = RPL * kCsrGroupCap + 8;  // room for the alignment slack
+   constexpr int NS = kCsrPatStages;
    __shared__ __align__( 16 ) Real sval[ kCsrGroupWarps ][ NS ][ SC ];
    __shared__ PatternSmem sp;
    if( sink.skip() )
@@ -606,35 +611,38 @@ csr_pattern_kernel( const int32_t* __restrict__ off, RowPatterns P, const Real* 
    const uint64_t pol = l2_evict_first();
    // this warp's groups start at rows row, row + step, ... (below 2^31 + step: kept unsigned)
    const unsigned end = (unsigned) row_end;
-   const unsigned step = gridDim.x * kCsrGroupWarps * kCsrGroupRows;
-   unsigned row = (unsigned) row_begin + ( blockIdx.x * kCsrGroupWarps + warp ) * kCsrGroupRows;
-   // this lane's row start and pattern in the group from g0 (dead lanes: the end of the last row)
-   auto load_row = [ & ]( unsigned g0, int& lo, int& p )
+   const unsigned step = gridDim.x * kCsrGroupWarps * kCsrGroupRows * RPL;
+   unsigned row = (unsigned) row_begin + ( blockIdx.x * kCsrGroupWarps + warp ) * kCsrGroupRows * RPL;
+   // this lane's row starts and patterns in the group from g0 (past the rows: the end of the last one)
+   auto load_row = [ & ]( unsigned g0, int( &lo )[ RPL ], int( &p )[ RPL ] )
    {
-      const unsigned r = min( g0 + lane, end );
-      lo = 0;
-      p = -1;
-      if( g0 < end ) {
-         lo = __ldg( off + r );
-         if( r < end )
-            p = __ldg( P.id + r );
+#pragma unroll
+      for( int j = 0; j < RPL; j++ ) {
+         const unsigned r = min( g0 + 32 * j + lane, end );
+         lo[ j ] = 0;
+         p[ j ] = -1;
+         if( g0 < end ) {
+            lo[ j ] = __ldg( off + r );
+            if( r < end )
+               p[ j ] = __ldg( P.id + r );
+         }
       }
    };
-   // the group's values: from lane 0's row start to the end of lane 31's row
-   auto stage = [ & ]( unsigned g0, int lo, int p, int buf )
+   // the group's values: from lane 0's first row start to the end of lane 31's last row
+   auto stage = [ & ]( unsigned g0, const int( &lo )[ RPL ], const int( &p )[ RPL ], int buf )
    {
       if( g0 < end ) {
-         const int len = p >= 0 ? sp.ptr[ p + 1 ] - sp.ptr[ p ] : 0;
-         const int v0 = __shfl_sync( 0xffffffffu, lo, 0 ) & ~( VPC - 1 );
-         const int n = __shfl_sync( 0xffffffffu, lo + len, 31 ) - v0;
+         const int q = p[ RPL - 1 ], len = q >= 0 ? sp.ptr[ q + 1 ] - sp.ptr[ q ] : 0;
+         const int v0 = __shfl_sync( 0xffffffffu, lo[ 0 ], 0 ) & ~( VPC - 1 );
+         const int n = __shfl_sync( 0xffffffffu, lo[ RPL - 1 ] + len, 31 ) - v0;
          const Real* src = val + v0;
          Real* dst = sval[ warp ][ buf ];
-         for( int q = VPC * lane; q < n; q += 32 * VPC )
-            cp_async16( dst + q, src + q, pol );
+         for( int c = VPC * lane; c < n; c += 32 * VPC )
+            cp_async16( dst + c, src + c, pol );
       }
       cp_async_commit();  // an empty group past the end keeps the wait counts uniform
    };
-   int lo[ NS ], pn[ NS ];
+   int lo[ NS ][ RPL ], pn[ NS ][ RPL ];
 #pragma unroll
    for( int i = 0; i < NS; i++ )
       load_row( row + i * step, lo[ i ], pn[ i ] );
@@ -646,45 +654,58 @@ csr_pattern_kernel( const int32_t* __restrict__ off, RowPatterns P, const Real* 
    int buf = 0;
    for( ; row < end; row += step ) {
       stage( row + ( NS - 1 ) * step, lo[ NS - 1 ], pn[ NS - 1 ], buf == 0 ? NS - 1 : buf - 1 );
-      int nlo, np;
+      int nlo[ RPL ], np[ RPL ];
       load_row( row + NS * step, nlo, np );
-      const int first = lo[ 0 ], p = pn[ 0 ];
-      const int pb = p >= 0 ? sp.ptr[ p ] : 0, len = p >= 0 ? sp.ptr[ p + 1 ] - pb : 0;
-      const int* so = sp.off + pb;
-      const Real* xr = x + ( row + lane );
-      // the gathers of the row's first elements need no column and go out
+      // the gathers of the rows' first elements need no column and go out
       // before the wait for the values
-      Real xv[ 8 ];
+      const int* so[ RPL ];
+      int len[ RPL ];
+      Real xv[ RPL ][ 8 ];
+      const Real* xr = x + ( row + lane );
 #pragma unroll
-      for( int i = 0; i < 8; i++ )
-         xv[ i ] = i < len ? __ldg( xr + so[ i ] ) : Real( 0 );
-      const Real* sv = sval[ warp ][ buf ] + ( first - ( __shfl_sync( 0xffffffffu, first, 0 ) & ~( VPC - 1 ) ) );
+      for( int j = 0; j < RPL; j++ ) {
+         const int p = pn[ 0 ][ j ], pb = p >= 0 ? sp.ptr[ p ] : 0;
+         len[ j ] = p >= 0 ? sp.ptr[ p + 1 ] - pb : 0;
+         so[ j ] = sp.off + pb;
+#pragma unroll
+         for( int i = 0; i < 8; i++ )
+            xv[ j ][ i ] = i < len[ j ] ? __ldg( xr + 32 * j + so[ j ][ i ] ) : Real( 0 );
+      }
+      const Real* sv = sval[ warp ][ buf ] - ( __shfl_sync( 0xffffffffu, lo[ 0 ][ 0 ], 0 ) & ~( VPC - 1 ) );
       cp_async_wait< NS - 1 >();  // this group's copies have landed
       __syncwarp();
-      Real sum = 0;
 #pragma unroll
-      for( int i = 0; i < 8; i++ )
-         if( i < len )
-            sum = sum + mul_rn( sv[ i ], xv[ i ] );
-      for( int k = 8; k < len; k += 8 ) {
+      for( int j = 0; j < RPL; j++ ) {
+         const Real* sr = sv + lo[ 0 ][ j ];
+         Real sum = 0;
 #pragma unroll
          for( int i = 0; i < 8; i++ )
-            xv[ i ] = k + i < len ? __ldg( xr + so[ k + i ] ) : Real( 0 );
+            if( i < len[ j ] )
+               sum = sum + mul_rn( sr[ i ], xv[ j ][ i ] );
+         for( int k = 8; k < len[ j ]; k += 8 ) {
+            Real xk[ 8 ];
 #pragma unroll
-         for( int i = 0; i < 8; i++ )
-            if( k + i < len )
-               sum = sum + mul_rn( sv[ k + i ], xv[ i ] );
+            for( int i = 0; i < 8; i++ )
+               xk[ i ] = k + i < len[ j ] ? __ldg( xr + 32 * j + so[ j ][ k + i ] ) : Real( 0 );
+#pragma unroll
+            for( int i = 0; i < 8; i++ )
+               if( k + i < len[ j ] )
+                  sum = sum + mul_rn( sr[ k + i ], xk[ i ] );
+         }
+         if( pn[ 0 ][ j ] >= 0 )
+            sink.put( (int) ( row + 32 * j + lane ), sum, acc.v );
       }
-      if( p >= 0 )
-         sink.put( (int) ( row + lane ), sum, acc.v );
       __syncwarp();  // the buffer is refilled NS groups later
 #pragma unroll
-      for( int i = 0; i < NS - 1; i++ ) {
-         lo[ i ] = lo[ i + 1 ];
-         pn[ i ] = pn[ i + 1 ];
+      for( int j = 0; j < RPL; j++ ) {
+#pragma unroll
+         for( int i = 0; i < NS - 1; i++ ) {
+            lo[ i ][ j ] = lo[ i + 1 ][ j ];
+            pn[ i ][ j ] = pn[ i + 1 ][ j ];
+         }
+         lo[ NS - 1 ][ j ] = nlo[ j ];
+         pn[ NS - 1 ][ j ] = np[ j ];
       }
-      lo[ NS - 1 ] = nlo;
-      pn[ NS - 1 ] = np;
       buf = buf + 1 == NS ? 0 : buf + 1;
    }
    cp_async_wait< 0 >();
@@ -1590,16 +1611,22 @@ constexpr int csr_group_rows_per_lane()
    return sizeof( Real ) == 4 ? B2S_CSR_GROUP_RPL_F32 : 1;
 }
 
-// grid of the row-group kernels on the rows [rb, re): the resident blocks only
-template< class Kernel >
+// grid of a row-group kernel on the rows [rb, re): the resident blocks only,
+// looked up once per kernel and device (this is on the path of every product)
+template< auto KERNEL >
 inline int
-csr_group_grid( Kernel kern, int32_t rb, int32_t re, int group_rows )
+csr_group_grid( int32_t rb, int32_t re, int group_rows )
 {
-   const int occ = resident_blocks( reinterpret_cast< const void* >( kern ), kCsrGroupBlock );
+   static int resident[ 64 ] = {};
+   const int dev = current_device();
+   int cap = dev >= 0 && dev < 64 ? resident[ dev ] : 0;
+   if( cap == 0 ) {
+      cap = std::min( num_sms() * resident_blocks( reinterpret_cast< const void* >( KERNEL ), kCsrGroupBlock ), kMaxReduceGrid );
+      if( dev >= 0 && dev < 64 )
+         resident[ dev ] = cap;
+   }
    const int64_t groups = ( (int64_t) re - rb + group_rows - 1 ) / group_rows;
-   const int64_t want = ( groups + kCsrGroupWarps - 1 ) / kCsrGroupWarps;
-   return (int) std::max< int64_t >( 1,
-                                     std::min< int64_t >( want, std::min< int64_t >( (int64_t) num_sms() * occ, kMaxReduceGrid ) ) );
+   return (int) std::min< int64_t >( ( groups + kCsrGroupWarps - 1 ) / kCsrGroupWarps, cap );
 }
 
 // the row-group kernel on the rows [rb, re) (rb a multiple of 32 RPL)
@@ -1608,9 +1635,8 @@ inline b2s_status
 launch_csr_group( const int32_t* off, const int32_t* col, const Real* values, const Real* x, int32_t rb, int32_t re,
                   const Sink& sink, RedScratch rs, cudaStream_t s )
 {
-   auto kern = csr_group_kernel< Real, RPL, Sink >;
-   kern<<< csr_group_grid( kern, rb, re, kCsrGroupRows * RPL ), kCsrGroupBlock, 0, s >>>( off, col, values, x, rb, re, sink,
-                                                                                         rs );
+   const int grid = csr_group_grid< csr_group_kernel< Real, RPL, Sink > >( rb, re, kCsrGroupRows * RPL );
+   csr_group_kernel< Real, RPL, Sink ><<< grid, kCsrGroupBlock, 0, s >>>( off, col, values, x, rb, re, sink, rs );
    B2S_TRY_CUDA( cudaGetLastError() );
    return B2S_OK;
 }
@@ -1649,9 +1675,9 @@ spmv_dispatch( const b2s_matrix_t* A, const Real* values, const Real* x, int32_t
       case B2S_CSR: {
          const int32_t* off = A->offsets.as< int32_t >();
          if( patterns && rb % kCsrGroupRows == 0 ) {
-            auto kern = csr_pattern_kernel< Real, Sink >;
-            kern<<< csr_group_grid( kern, rb, re, kCsrGroupRows ), kCsrGroupBlock, 0, s >>>( off, A->patterns(), values, x, rb,
-                                                                                           re, sink, rs );
+            const int grid = csr_group_grid< csr_pattern_kernel< Real, Sink > >( rb, re, kCsrGroupRows * kCsrPatRows );
+            csr_pattern_kernel< Real, Sink ><<< grid, kCsrGroupBlock, 0, s >>>( off, A->patterns(), values, x, rb, re, sink,
+                                                                               rs );
             break;
          }
          if( A->csr_kernel == B2S_CSR_ADAPTIVE && A->csr_group && rb % kCsrGroupRows == 0 ) {
