@@ -1,0 +1,66 @@
+"""Handles that are used again after their matrix was permuted in place: what
+was captured with the arrays' old addresses must not run again. Each result
+equals, bit for bit, that of a handle made after the permutation."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+N = 110_000  # above the row count from which products go through row patterns
+
+
+def _band(offsets, seed):
+    g = np.random.default_rng(seed)
+    i = np.arange(N)
+    c = i[:, None] + np.asarray(offsets)[None, :]
+    keep = (c >= 0) & (c < N)
+    val = g.uniform(-1, 1, c.shape)
+    val[:, list(offsets).index(0)] = 2.0 * len(offsets)
+    off = np.concatenate([[0], np.cumsum(keep.sum(axis=1))]).astype(np.int32)
+    return off, c[keep].astype(np.int32), val[keep]
+
+
+def _same_bits(cuda, a, b):
+    return cuda.equal(a.view(cuda.int64), b.view(cuda.int64))
+
+
+PERMUTATIONS = {
+    # patterns before and after, of other rows
+    "roll": lambda: np.roll(np.arange(N), 3),
+    # more patterns than are kept: the columns are read again
+    "random": lambda: np.random.default_rng(1).permutation(N),
+}
+
+
+def _permute(M, where, name):
+    p = PERMUTATIONS[name]().astype(np.int32)
+    (M.permuteColumns if where == "columns" else M.permuteRows)(p)
+
+
+@pytest.mark.parametrize("where,segments", [("columns", "CSR"), ("columns", "SlicedEllpack"), ("columns", "BiEllpack"),
+                                            ("rows", "CSR")])
+@pytest.mark.parametrize("name", list(PERMUTATIONS))
+@pytest.mark.parametrize("solver", ["GMRES", "TFQMR"])
+def test_solver_used_again(b2s_lib, cuda, where, segments, name, solver):
+    csr = _band([-400, -1, 0, 1, 400], 3)
+    M = b2s_lib.SparseMatrix.from_csr(*csr, N, segments=segments)
+    b = cuda.rand(N, dtype=cuda.float64, device="cuda")
+
+    def solve(s):
+        x = cuda.zeros_like(b)
+        s.solve(b, x)
+        return x
+
+    def make():
+        s = getattr(b2s_lib, solver)()
+        s.setMatrix(M)
+        s.setConvergenceResidue(1e-10)
+        s.setMaxIterations(12)  # permuted, the system need not converge
+        return s
+
+    s = make()
+    before = solve(s)
+    _permute(M, where, name)
+    again = solve(s)
+    assert not _same_bits(cuda, again, before)
+    assert _same_bits(cuda, again, solve(make()))

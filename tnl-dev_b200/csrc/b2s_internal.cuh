@@ -196,6 +196,9 @@ struct b2s_matrix_t
    int64_t storage = 0;       // TNL getStorageSize()
    int64_t alloc_elems = 0;   // slots allocated on the device (BiEllpack: only the addressed part)
    int device = 0;
+   // counts the changes in place (permutations), after which arrays may lie at
+   // other addresses: a graph captured with them holds for one generation
+   uint64_t generation = 0;
 
    b2s::DevBuf values, columns;
    b2s::DevBuf values32;      // optional FP32 copy (mixed precision inner solves)

@@ -826,17 +826,26 @@ struct b2s_solver_t
    int64_t ld = 0;
    int mmax = 0;
 
+   // captured with the addresses of A's arrays: valid for one generation of A
    std::map< long long, cudaGraphExec_t > graphs;
    std::map< long long, cudaGraph_t > graph_defs;
+   uint64_t generation = 0;
    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
    std::chrono::steady_clock::time_point t_start;
 
-   ~b2s_solver_t()
+   void drop_graphs()
    {
       for( auto& kv : graphs )
          cudaGraphExecDestroy( kv.second );
       for( auto& kv : graph_defs )
          cudaGraphDestroy( kv.second );
+      graphs.clear();
+      graph_defs.clear();
+   }
+
+   ~b2s_solver_t()
+   {
+      drop_graphs();
       if( h_ctl && h_ctl_pinned )
          cudaFreeHost( h_ctl );
       else
@@ -2652,6 +2661,7 @@ b2s_solver_create( b2s_matrix A, const b2s_solve_opts* opts, b2s_solver* out )
    S->o = o;
    S->mixed = o.precision == B2S_PRECISION_MIXED;
    S->n = A->rows;
+   S->generation = A->generation;
    const AllocCtx* actx = thread_alloc_ctx();
    if( actx && actx->solver_stream ) {
       S->cs = actx->solver_stream;
@@ -2762,6 +2772,10 @@ b2s_solve( b2s_solver S, const void* b, void* x, b2s_memory where, b2s_stream st
    const int64_t n = S->n;
    cudaStream_t us = as_stream( stream );
    S->t_start = std::chrono::steady_clock::now();
+   if( S->generation != S->A->generation ) {
+      S->drop_graphs();
+      S->generation = S->A->generation;
+   }
    // order the solver's private stream after the caller's stream
    B2S_TRY_CUDA( cudaEventRecord( S->ev0, us ) );
    B2S_TRY_CUDA( cudaStreamWaitEvent( S->cs, S->ev0, 0 ) );

@@ -205,7 +205,9 @@ b2s_matrix_permute_rows( b2s_matrix A, const int32_t* perm, b2s_memory where, b2
    // the permuted matrix takes the place of A (same handle for the caller)
    std::unique_ptr< b2s_matrix_t > hold( tmp );
    B2S_TRY_CUDA( cudaStreamSynchronize( s ) );
+   const uint64_t generation = A->generation + 1;
    *A = std::move( *tmp );
+   A->generation = generation;
    return B2S_OK;
 }
 
@@ -232,6 +234,7 @@ b2s_matrix_permute_columns( b2s_matrix A, const int32_t* iperm, b2s_memory where
       perm_columns_kernel<<< pgrid( A->alloc_elems ), 256, 0, s >>>( A->columns.as< int32_t >(), A->alloc_elems, dp );
       B2S_TRY_CUDA( cudaGetLastError() );
    }
+   A->generation++;
    // the Jacobi diagonal follows the new column indices
    B2S_TRY( build_diagonal( A, s ) );
    B2S_TRY( build_row_patterns( A, s ) );
