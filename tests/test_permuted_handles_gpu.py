@@ -64,3 +64,23 @@ def test_solver_used_again(b2s_lib, cuda, where, segments, name, solver):
     again = solve(s)
     assert not _same_bits(cuda, again, before)
     assert _same_bits(cuda, again, solve(make()))
+
+
+@pytest.mark.parametrize("name", list(PERMUTATIONS))
+@pytest.mark.parametrize("pinned", [True, False])
+def test_host_products_used_again(b2s_lib, cuda, name, pinned):
+    """Host vectors go through a pipeline whose schedule follows the columns
+    (page-locked ones through a captured graph)."""
+    M = b2s_lib.SparseMatrix.from_csr(*_band([-400, -1, 0, 1, 400], 4), N)
+    x = cuda.rand(N, dtype=cuda.float64)
+    y = cuda.zeros(N, dtype=cuda.float64)
+    if pinned:
+        x, y = x.pin_memory(), y.pin_memory()
+    M.vectorProduct(x, y)
+    _permute(M, "columns", name)
+    want = cuda.zeros(N, dtype=cuda.float64, device="cuda")
+    M.vectorProduct(x.cuda(), want)
+    for _ in range(2):
+        y.fill_(float("nan"))
+        M.vectorProduct(x, y)
+        assert _same_bits(cuda, y, want.cpu())

@@ -235,6 +235,7 @@ b2s_matrix_permute_columns( b2s_matrix A, const int32_t* iperm, b2s_memory where
       B2S_TRY_CUDA( cudaGetLastError() );
    }
    A->generation++;
+   A->pipe.reset();  // its graph reads the patterns, its row cuts follow the columns
    // the Jacobi diagonal follows the new column indices
    B2S_TRY( build_diagonal( A, s ) );
    B2S_TRY( build_row_patterns( A, s ) );
