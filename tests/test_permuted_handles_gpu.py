@@ -84,3 +84,23 @@ def test_host_products_used_again(b2s_lib, cuda, name, pinned):
         y.fill_(float("nan"))
         M.vectorProduct(x, y)
         assert _same_bits(cuda, y, want.cpu())
+
+
+@pytest.mark.parametrize("where", ["columns", "rows"])
+@pytest.mark.parametrize("longest", [6, 400])  # substitutions by blocks and a warp per row
+def test_factors_used_again(b2s_lib, cuda, where, longest):
+    """ILU(0) factors are those of the matrix at the time they were made."""
+    n, g = 3000, np.random.default_rng(8)
+    cols = [np.unique(np.concatenate([[i], g.integers(0, n, g.integers(0, longest + 1))])) for i in range(n)]
+    off = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.int32)
+    col = np.concatenate(cols).astype(np.int32)
+    val = g.uniform(-1, 1, len(col))
+    val[col == np.repeat(np.arange(n), np.diff(off))] = 2.0 * longest + 4.0
+    M = b2s_lib.SparseMatrix.from_csr(off, col, val, n)
+    P = b2s_lib.Preconditioner(M, "ilu0")
+    b = cuda.rand(n, dtype=cuda.float64, device="cuda")
+    before, after = cuda.zeros_like(b), cuda.zeros_like(b)
+    P.solve(b, before)
+    (M.permuteColumns if where == "columns" else M.permuteRows)(g.permutation(n).astype(np.int32))
+    P.solve(b, after)
+    assert _same_bits(cuda, before, after)

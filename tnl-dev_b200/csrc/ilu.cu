@@ -311,6 +311,20 @@ ilu_factorize( const b2s_matrix_t* A, const Real* values, IluFactors< Real >& F,
    ilu_factor_kernel< Real ><<< F.grid, kIluBlock, 0, s >>>( v );
    B2S_TRY_CUDA( cudaGetLastError() );
    B2S_TRY( ilu_pack( F, s ) );
+   if( F.off == A->offsets.template as< int32_t >() ) {
+      // the matrix may be permuted in place: the factors keep no pointer into it
+      F.off = F.col = nullptr;
+      if( F.blocks == 0 ) {  // the warp-per-row kernel reads the pattern
+         B2S_TRY( F.off_own.alloc( ( (size_t) n + 1 ) * sizeof( int32_t ) ) );
+         B2S_TRY( F.col_own.alloc( (size_t) std::max< int64_t >( nnz, 1 ) * sizeof( int32_t ) ) );
+         B2S_TRY_CUDA( cudaMemcpyAsync( F.off_own.p, A->offsets.p, ( (size_t) n + 1 ) * sizeof( int32_t ),
+                                        cudaMemcpyDeviceToDevice, s ) );
+         B2S_TRY_CUDA( cudaMemcpyAsync( F.col_own.p, A->columns.p, (size_t) nnz * sizeof( int32_t ),
+                                        cudaMemcpyDeviceToDevice, s ) );
+         F.off = F.off_own.template as< int32_t >();
+         F.col = F.col_own.template as< int32_t >();
+      }
+   }
    B2S_TRY_CUDA( cudaStreamSynchronize( s ) );
    return F.check( s );
 }
