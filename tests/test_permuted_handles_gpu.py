@@ -40,7 +40,7 @@ def _permute(M, where, name):
 @pytest.mark.parametrize("where,segments", [("columns", "CSR"), ("columns", "SlicedEllpack"), ("columns", "BiEllpack"),
                                             ("rows", "CSR")])
 @pytest.mark.parametrize("name", list(PERMUTATIONS))
-@pytest.mark.parametrize("solver", ["GMRES", "TFQMR"])
+@pytest.mark.parametrize("solver", ["GMRES", "TFQMR", "SOR"])
 def test_solver_used_again(b2s_lib, cuda, where, segments, name, solver):
     csr = _band([-400, -1, 0, 1, 400], 3)
     M = b2s_lib.SparseMatrix.from_csr(*csr, N, segments=segments)

@@ -2552,6 +2552,15 @@ solve_mixed( b2s_solver_t* S, b2s_solve_report& rep )
    return mixed_refine( S, rep );
 }
 
+// the SOR sweep's level order, once per solver and state of the matrix
+static b2s_status
+build_sor_plan( b2s_solver_t* S )
+{
+   if( S->A->dtype == B2S_F64 )
+      return S->sor64.build( S->A, S->cs );
+   return S->sor32.build( S->A, S->cs );
+}
+
 template< typename Real >
 __global__ void
 cast_vec_kernel( const Real* __restrict__ in, float* __restrict__ out, int64_t n )
@@ -2729,13 +2738,8 @@ b2s_solver_create( b2s_matrix A, const b2s_solve_opts* opts, b2s_solver* out )
       B2S_TRY( S->V.alloc( (size_t) ( M + 1 ) * S->ld * es ) );
       B2S_TRY( S->gm.alloc( (size_t) ( ( M + 1 ) * M + 5 * ( M + 1 ) ) * sizeof( double ) ) );
    }
-   if( o.solver == B2S_SOR ) {
-      // the sweep's level order, once per solver
-      if( A->dtype == B2S_F64 )
-         B2S_TRY( S->sor64.build( A, S->cs ) );
-      else
-         B2S_TRY( S->sor32.build( A, S->cs ) );
-   }
+   if( o.solver == B2S_SOR )
+      B2S_TRY( build_sor_plan( S.get() ) );
    if( o.solver == B2S_BICGSTABL ) {
       // R and U, ell + 1 columns each (BICGStabL.hpp:280-285), and T, sigma, g_0..g_2
       const int ell = o.bicgstab_ell;
@@ -2774,6 +2778,8 @@ b2s_solve( b2s_solver S, const void* b, void* x, b2s_memory where, b2s_stream st
    S->t_start = std::chrono::steady_clock::now();
    if( S->generation != S->A->generation ) {
       S->drop_graphs();
+      if( S->o.solver == B2S_SOR )  // the sweep's plan points into A
+         B2S_TRY( build_sor_plan( S ) );
       S->generation = S->A->generation;
    }
    // order the solver's private stream after the caller's stream
