@@ -462,6 +462,36 @@ batch_diag_kernel( int64_t rows, const int32_t* __restrict__ off, const int32_t*
    }
 }
 
+// The first row whose offsets do not lie in [0, nnz] in order or that has a
+// column outside its system's diagonal block: solve_system turns columns into
+// places of the system's vectors, in another CTA's shared memory among others.
+__global__ void
+batch_check_kernel( int64_t rows, int64_t nnz, int nsys, const int64_t* __restrict__ row_ptr,
+                    const int32_t* __restrict__ off, const int32_t* __restrict__ col, int* bad )
+{
+   for( int64_t r = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; r < rows; r += (int64_t) gridDim.x * blockDim.x ) {
+      const int b = off[ r ], e = off[ r + 1 ];
+      if( b < 0 || e < b || e > nnz ) {
+         atomicMin( bad, (int) r );
+         continue;
+      }
+      int lo = 0, hi = nsys;  // the last system that starts at or before r (empty ones start there too)
+      while( hi - lo > 1 ) {
+         const int mid = ( lo + hi ) / 2;
+         if( row_ptr[ mid ] <= r )
+            lo = mid;
+         else
+            hi = mid;
+      }
+      const int64_t c0 = row_ptr[ lo ], c1 = row_ptr[ lo + 1 ];
+      for( int t = b; t < e; t++ )
+         if( col[ t ] < c0 || col[ t ] >= c1 ) {
+            atomicMin( bad, (int) r );
+            break;
+         }
+   }
+}
+
 }  // namespace b2s
 
 using namespace b2s;
@@ -688,6 +718,23 @@ b2s_batch_create( int32_t nsys, const int64_t* row_ptr, const int32_t* nrhs, con
       B2S_TRY_CUDA( cudaMemcpyAsync( bt->col.p, columns, bt->nnz * sizeof( int32_t ), kin, s ) );
       B2S_TRY_CUDA( cudaMemcpyAsync( bt->val.p, values, bt->nnz * sizeof( double ), kin, s ) );
    }
+   B2S_TRY( bt->row_ptr.alloc( ( nsys + 1 ) * sizeof( int64_t ) ) );
+   B2S_TRY( copy_h2d( bt->row_ptr.p, bt->row_ptr_h.data(), ( nsys + 1 ) * sizeof( int64_t ), s ) );
+   if( bt->rows > 0 ) {
+      B2S_TRY( bt->counter.alloc( 64 ) );
+      const int none = INT32_MAX;
+      B2S_TRY( copy_h2d( bt->counter.p, &none, sizeof( int ), s ) );
+      batch_check_kernel<<< (int) std::min< int64_t >( ( bt->rows + 255 ) / 256, (int64_t) num_sms() * 16 ), 256, 0,
+                               s >>>( bt->rows, bt->nnz, nsys, bt->row_ptr.as< int64_t >(), bt->off.as< int32_t >(),
+                                      bt->col.as< int32_t >(), bt->counter.as< int >() );
+      B2S_TRY_CUDA( cudaGetLastError() );
+      int bad = none;
+      B2S_TRY( copy_d2h( &bad, bt->counter.p, sizeof( int ), s ) );
+      if( bad != none ) {
+         set_error( "batch: row %d has offsets out of order or a column outside its system's block", bad );
+         return B2S_INVALID_ARG;
+      }
+   }
    B2S_TRY( bt->diag.alloc( std::max< int64_t >( bt->rows, 1 ) * sizeof( double ) ) );
    if( bt->rows > 0 ) {
       batch_diag_kernel<<< (int) std::min< int64_t >( ( bt->rows + 255 ) / 256, (int64_t) num_sms() * 16 ), 256, 0,
@@ -695,12 +742,10 @@ b2s_batch_create( int32_t nsys, const int64_t* row_ptr, const int32_t* nrhs, con
                                      bt->diag.as< double >() );
       B2S_TRY_CUDA( cudaGetLastError() );
    }
-   B2S_TRY( bt->row_ptr.alloc( ( nsys + 1 ) * sizeof( int64_t ) ) );
    B2S_TRY( bt->nrhs.alloc( std::max( nsys, 1 ) * sizeof( int32_t ) ) );
    B2S_TRY( bt->vec_off.alloc( std::max( nsys, 1 ) * sizeof( int64_t ) ) );
    B2S_TRY( bt->rhs_off.alloc( std::max( nsys, 1 ) * sizeof( int64_t ) ) );
    B2S_TRY( bt->order.alloc( std::max( nsys, 1 ) * sizeof( int32_t ) ) );
-   B2S_TRY( copy_h2d( bt->row_ptr.p, bt->row_ptr_h.data(), ( nsys + 1 ) * sizeof( int64_t ), s ) );
    if( nsys > 0 ) {
       B2S_TRY( copy_h2d( bt->nrhs.p, bt->nrhs_h.data(), nsys * sizeof( int32_t ), s ) );
       B2S_TRY( copy_h2d( bt->vec_off.p, bt->vec_off_h.data(), nsys * sizeof( int64_t ), s ) );
@@ -711,7 +756,8 @@ b2s_batch_create( int32_t nsys, const int64_t* row_ptr, const int32_t* nrhs, con
    B2S_TRY( bt->R.alloc( vb ) );
    B2S_TRY( bt->P.alloc( vb ) );
    B2S_TRY( bt->AP.alloc( vb ) );
-   B2S_TRY( bt->counter.alloc( 64 ) );
+   if( ! bt->counter.p )
+      B2S_TRY( bt->counter.alloc( 64 ) );
    B2S_TRY( bt->it_out.alloc( std::max< int64_t >( bt->nslots, 1 ) * sizeof( int64_t ) ) );
    B2S_TRY( bt->res_out.alloc( std::max< int64_t >( bt->nslots, 1 ) * sizeof( double ) ) );
    B2S_TRY( bt->status_out.alloc( std::max< int64_t >( bt->nslots, 1 ) * sizeof( int32_t ) ) );
