@@ -3,8 +3,8 @@
 
 Patterns where a block plan can go wrong: one row, sizes around a batch of 32
 rows and around one block, chains (one row per level), rows of no, few and
-many entries, dependencies on far blocks, and rows too long for a lane (the
-warp-per-row kernel)."""
+many entries, dependencies on far blocks, and rows too long for a lane or too
+uneven for a batch (the warp-per-row kernel)."""
 import numpy as np
 import pytest
 
@@ -33,15 +33,30 @@ def _random(n, longest, seed):
     return off, col, val, n
 
 
+def _uneven(n):
+    """Rows past the first 128 depend on row 0, every 32nd of them on rows 0 to 99 too."""
+    cols = [np.arange(100 if i % 32 == 0 else 1) for i in range(n)]
+    cols = [np.array([i]) if i < 128 else np.append(c, i) for i, c in enumerate(cols)]
+    off = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.int32)
+    col = np.concatenate(cols).astype(np.int32)
+    val = np.random.default_rng(5).uniform(-1, 1, len(col))
+    val[off[1:] - 1] = 200.0
+    return off, col, val, n
+
+
 CASES = {
     "one_row": lambda: _band(1, []),
     "diagonal": lambda: _band(70, []),
     "chain_31": lambda: _band(31, [-1, 1]),
-    "chain_5000": lambda: _band(5000, [-1, 1]),  # a level per row, across blocks
+    "chain_5000": lambda: _band(5000, [-1, 1]),  # a level per row
+    "chain_20000": lambda: _band(20000, [-1, 1]),  # and across three blocks
+    "narrow_17000": lambda: _band(17000, [-3, -1, 1, 3]),  # a few rows per level and block
     "far_8193": lambda: _band(8193, [-4096, -1, 1, 4096, 8000]),
     "grid_4097": lambda: _band(4097, [-64, -1, 1, 64]),
     "random_short": lambda: _random(20000, 6, 1),
     "random_ragged": lambda: _random(9000, 40, 2),
+    # a row of 100 among 31 of one entry in every batch
+    "uneven": lambda: _uneven(4096),
     "long_rows": lambda: _random(3000, 400, 3),  # the warp-per-row kernel
 }
 
@@ -81,3 +96,27 @@ def test_block_substitutions_not_a_number(b2s_lib, cuda):
     x = cuda.zeros_like(b)
     P.solve(b, x)
     assert bool(cuda.isnan(x).all())
+
+
+def test_memory_of_a_chain(b2s_lib, cuda, oracle):
+    """One row per level: the plans of both triangles stay near the factors' size."""
+    n = 400_000
+    g = np.random.default_rng(2)
+    i = np.repeat(np.arange(n), 3).reshape(n, 3) + np.array([-1, 0, 1])
+    keep = (i >= 0) & (i < n)
+    off = np.concatenate([[0], np.cumsum(keep.sum(axis=1))]).astype(np.int32)
+    val = g.uniform(-1, 1, i.shape)
+    val[:, 1] = 4.0
+    csr = (off, i[keep].astype(np.int32), val[keep], n)
+    A = b2s_lib.SparseMatrix.from_csr(*csr[:3], n)
+    cuda.cuda.synchronize()
+    before = cuda.cuda.mem_get_info()[0]
+    P = b2s_lib.Preconditioner(A, "ilu0")
+    held = before - cuda.cuda.mem_get_info()[0]
+    # per row: 3 values of the factors, position of the diagonal, flag, order, two scratch values (52 bytes),
+    # and in each plan a batch (16), row, length, diagonal (16) and one slot (12): 140 bytes
+    assert held <= 160 * n + (48 << 20), held / n  # allocations take whole 2 MB pages
+    b = g.uniform(-1, 1, n)
+    x = cuda.zeros(n, dtype=cuda.float64, device="cuda")
+    P.solve(cuda.tensor(b, device="cuda"), x)
+    assert np.array_equal(x.cpu().numpy(), oracle.ilu0_apply(csr, b, "f64"))

@@ -74,6 +74,14 @@ choose_blocks( IluFactors< Real >& F, const std::vector< int32_t >& hoff )
    F.blocks = ( n + rows - 1 ) / rows;
 }
 
+// A batch takes the slots of its longest row for all of its rows: a factor
+// whose rows differ so much that this is more than kTrsvMaxPadding slots per
+// entry takes a warp per row.
+constexpr int64_t kTrsvMaxPadding = 4;
+// Batches of 32 lanes each up to this many lanes per row and slots per slot in
+// use (see FULL).
+constexpr int64_t kTrsvFullLanes = 3;
+
 // One triangle's batches: the rows of each block by level, cut into batches of
 // up to 32 rows of one level. deps( i ): row i's entries in this triangle.
 template< typename Real, class Deps >
@@ -81,15 +89,17 @@ static b2s_status
 block_plan( IluFactors< Real >& F, TrsvPlan< Real >& P, const std::vector< int32_t >& lev, Deps deps, cudaStream_t s )
 {
    const int32_t G = F.blocks, R = F.rows_per_block;
-   std::vector< int32_t > first( (size_t) G + 1, 0 ), row, width, order, count;
-   row.reserve( (size_t) F.n + (size_t) F.n / 4 );
+   std::vector< int32_t > first( (size_t) G + 1, 0 ), row( (size_t) F.n ), count;
+   std::vector< int4 > batch;
+   batch.reserve( (size_t) F.n / 16 + (size_t) G );
+   int64_t slots = 0, entries = 0;
    for( int32_t c = 0; c < G; c++ ) {
       const int32_t r0 = c * R, r1 = std::min( F.n, r0 + R );
       const auto range = std::minmax_element( lev.begin() + r0, lev.begin() + r1 );
       const int32_t lo = *range.first;
       const int64_t span = (int64_t) *range.second - lo + 1;
       // the block's rows by level, in increasing order within one
-      order.resize( (size_t) ( r1 - r0 ) );
+      int32_t* order = row.data() + r0;
       if( span <= 8LL * R ) {
          count.assign( (size_t) span + 1, 0 );
          for( int32_t i = r0; i < r1; i++ )
@@ -102,44 +112,56 @@ block_plan( IluFactors< Real >& F, TrsvPlan< Real >& P, const std::vector< int32
       else {
          for( int32_t i = r0; i < r1; i++ )
             order[ i - r0 ] = i;
-         std::stable_sort( order.begin(), order.end(), [ & ]( int32_t x, int32_t y ) { return lev[ x ] < lev[ y ]; } );
+         std::stable_sort( order, order + ( r1 - r0 ), [ & ]( int32_t x, int32_t y ) { return lev[ x ] < lev[ y ]; } );
       }
-      int32_t fill = 32, level = -1;
-      for( const int32_t i : order ) {
-         if( fill == 32 || level != lev[ i ] ) {
-            row.resize( width.size() * 32, -1 );
-            width.push_back( 0 );
-            fill = 0;
+      int32_t level = -1;
+      for( int32_t k = r0; k < r1; k++ ) {
+         const int32_t i = row[ k ], d = deps( i );
+         if( level != lev[ i ] || batch.back().z == 32 ) {
+            batch.push_back( make_int4( k, 0, 0, 0 ) );
             level = lev[ i ];
          }
-         row.push_back( i );
-         fill++;
-         width.back() = std::max( width.back(), deps( i ) );
+         int4& h = batch.back();
+         h.z++;
+         h.w = std::max( h.w, d );
+         entries += d;
       }
-      row.resize( width.size() * 32, -1 );
-      first[ c + 1 ] = (int32_t) width.size();
+      first[ c + 1 ] = (int32_t) batch.size();
    }
    P.batches = first[ G ];
-   width.push_back( 0 );
-   int64_t slots = 0;
-   for( int32_t q = 0; q <= P.batches; q++ ) {
-      const int32_t w = width[ q ];
-      width[ q ] = (int32_t) slots;
-      slots += w;
+   int64_t wide = 0;  // slots of batches of 32 lanes
+   for( const int4& h : batch ) {
+      slots += (int64_t) h.z * h.w;
+      wide += 32LL * h.w;
    }
-   if( slots > INT32_MAX / 64 ) {  // padded slots past int32: warp per row
+   if( slots > kTrsvMaxPadding * std::max< int64_t >( entries, F.n ) || slots > INT32_MAX / 2 ) {
       F.blocks = 0;
       return B2S_OK;
    }
+   P.full = 32LL * P.batches <= kTrsvFullLanes * F.n && wide <= kTrsvFullLanes * slots && wide <= INT32_MAX / 2;
+   if( P.full ) {
+      std::vector< int32_t > lanes( (size_t) P.batches * 32, -1 );
+      for( size_t q = 0; q < batch.size(); q++ ) {
+         std::copy_n( row.begin() + batch[ q ].x, batch[ q ].z, lanes.begin() + (ptrdiff_t) ( 32 * q ) );
+         batch[ q ].x = (int32_t) ( 32 * q );
+         batch[ q ].z = 32;
+      }
+      row.swap( lanes );
+   }
+   slots = 0;
+   for( int4& h : batch ) {
+      h.y = (int32_t) slots;
+      slots += (int64_t) h.z * h.w;
+   }
    B2S_TRY( P.bfirst.alloc( first.size() * sizeof( int32_t ) ) );
-   B2S_TRY( P.bptr.alloc( width.size() * sizeof( int32_t ) ) );
+   B2S_TRY( P.batch.alloc( batch.size() * sizeof( int4 ) ) );
    B2S_TRY( P.row.alloc( row.size() * sizeof( int32_t ) ) );
    B2S_TRY( P.len.alloc( row.size() * sizeof( int32_t ) ) );
    B2S_TRY( P.dg.alloc( row.size() * sizeof( Real ) ) );
-   B2S_TRY( P.col.alloc( (size_t) std::max< int64_t >( slots, 1 ) * 32 * sizeof( int32_t ) ) );
-   B2S_TRY( P.val.alloc( (size_t) std::max< int64_t >( slots, 1 ) * 32 * sizeof( Real ) ) );
+   B2S_TRY( P.col.alloc( (size_t) std::max< int64_t >( slots, 1 ) * sizeof( int32_t ) ) );
+   B2S_TRY( P.val.alloc( (size_t) std::max< int64_t >( slots, 1 ) * sizeof( Real ) ) );
    B2S_TRY( copy_h2d( P.bfirst.p, first.data(), first.size() * sizeof( int32_t ), s ) );
-   B2S_TRY( copy_h2d( P.bptr.p, width.data(), width.size() * sizeof( int32_t ), s ) );
+   B2S_TRY( copy_h2d( P.batch.p, batch.data(), batch.size() * sizeof( int4 ), s ) );
    return copy_h2d( P.row.p, row.data(), row.size() * sizeof( int32_t ), s );
 }
 
@@ -153,11 +175,11 @@ ilu_pack( IluFactors< Real >& F, cudaStream_t s )
    B2S_TRY( F.clear_scratch( s ) );
    const TrsvPlan< Real >&l = F.plan_l, &u = F.plan_u;
    trsv_pack_kernel< Real, false ><<< grid_n( 32LL * l.batches ), 256, 0, s >>>(
-      32 * l.batches, l.row.template as< int32_t >(), l.bptr.template as< int32_t >(), F.off,
+      l.batches, l.batch.template as< int4 >(), l.row.template as< int32_t >(), F.off,
       F.diag.template as< int32_t >(), F.col, F.lu.template as< Real >(), l.len.template as< int32_t >(),
       l.col.template as< int32_t >(), l.val.template as< Real >(), l.dg.template as< Real >() );
    trsv_pack_kernel< Real, true ><<< grid_n( 32LL * u.batches ), 256, 0, s >>>(
-      32 * u.batches, u.row.template as< int32_t >(), u.bptr.template as< int32_t >(), F.off,
+      u.batches, u.batch.template as< int4 >(), u.row.template as< int32_t >(), F.off,
       F.diag.template as< int32_t >(), F.col, F.lu.template as< Real >(), u.len.template as< int32_t >(),
       u.col.template as< int32_t >(), u.val.template as< Real >(), u.dg.template as< Real >() );
    B2S_TRY_CUDA( cudaGetLastError() );
@@ -220,8 +242,10 @@ ilu_levels( IluFactors< Real >& F, const std::vector< int32_t >& hoff, const std
    F.levels_u = depth;
    if( F.blocks > 0 )
       B2S_TRY( block_plan< Real >( F, F.plan_u, lev, [ & ]( int32_t i ) { return hoff[ i + 1 ] - hdiag[ i ] - 1; }, s ) );
-   if( F.blocks == 0 )  // U's order serves the warp-per-row kernel only (L's the factorization too)
-      B2S_TRY( order( depth, F.ord_u, F.n_ord_u ) );
+   if( F.blocks == 0 ) {
+      F.plan_l = TrsvPlan< Real >();  // made before U's rows turned out not to suit
+      B2S_TRY( order( depth, F.ord_u, F.n_ord_u ) );  // for the warp-per-row kernel (L's also for the factorization)
+   }
    // resident warps only: every SM full of 256-thread blocks
    F.grid = num_sms() * ( 2048 / kIluBlock );
    return B2S_OK;

@@ -281,7 +281,11 @@ ilu_trsv_kernel( IluView< Real > L, const Real* b, Real* x )
 //     turn it is. The first look at other blocks' rows goes out before that.
 //   * A batch's columns, values and diagonal are stored batch by batch in slot
 //     order, so a warp loads them coalesced, one and two batches ahead of the
-//     one whose turn it is.
+//     one whose turn it is. Where most lanes have a row, batches are stored 32
+//     lanes wide (FULL); where few rows share a level, which would take up to 32
+//     times the entries, with as many lanes as they have rows. The latter takes
+//     a few more instructions and one more load in a row, per batch; both
+//     substitutions of 10^3 50 / 55 us, 64^3 282 / 285 us.
 //   * Blocks are claimed in dependency order from a ticket counter: a claimed
 //     block waits only for blocks claimed before it, whose CTAs are running.
 //     The CTA that takes the last ticket puts the counter back.
@@ -365,15 +369,15 @@ struct TrsvView
 {
    int32_t n, rows_per_block;
    const int32_t* bfirst;  // first batch of each block (blocks + 1 entries)
-   const int32_t* bptr;    // first slot of each batch / 32 (batches + 1 entries)
-   const int32_t* row;     // row of each lane of each batch, -1: none
-   const int32_t* len;     // its dependencies
-   const int32_t* col;     // slot k of lane l of a batch at ( bptr + k ) * 32 + l
+   const int4* batch;      // x: place of a batch's first lane, y: its first slot, z: lanes, w: slots per lane
+   const int32_t* row;     // rows in batch order (-1: a lane without one)
+   const int32_t* len;     // their dependencies
+   const int32_t* col;     // slot k of lane l of a batch at y + k * z + l
    const Real* val;
-   const Real* dg;         // U_ii of each lane of each batch (upper only)
+   const Real* dg;         // U_ii of the rows in batch order (upper only)
 };
 
-template< typename Real, bool UPPER, bool PLAIN, class Gate >
+template< typename Real, bool UPPER, bool PLAIN, bool FULL, class Gate >
 __global__ void __launch_bounds__( kTrsvBlock, 1 )
 ilu_block_trsv_kernel( TrsvView< Real > T, IluState* st, const Real* b, typename TrsvBits< Real >::type* pub,
                        typename TrsvBits< Real >::type* other, Real* x, Gate gate )
@@ -403,11 +407,11 @@ ilu_block_trsv_kernel( TrsvView< Real > T, IluState* st, const Real* b, typename
    __syncthreads();
    const int last = T.bfirst[ blk + 1 ];
    bool ok = true;  // false once a wait gave up: no more waits, the count goes on
-   // a batch's lane: loaded two batches (meta) and one batch (slots, right-hand
-   // side) ahead of its turn, so that no turn waits for them
+   // a batch's lane: loaded three batches (head; two if FULL), two (meta) and one
+   // (slots, right-hand side) ahead of its turn, so that no turn waits for them
    struct Meta
    {
-      int row, len, ptr, width;
+      int row, len, slot, rows, width;
       Real dg;
    };
    struct Slots
@@ -415,34 +419,41 @@ ilu_block_trsv_kernel( TrsvView< Real > T, IluState* st, const Real* b, typename
       Real b, val[ kTrsvSlots ];
       int col[ kTrsvSlots ];
    };
-   auto load_meta = [ & ]( int q )
+   auto load_head = [ & ]( int q ) { return q < last ? __ldg( T.batch + q ) : make_int4( 0, 0, 0, 0 ); };
+   auto load_meta = [ & ]( int q, const int4& head )
    {
-      Meta m{ -1, 0, 0, 0, Real( 1 ) };
-      if( q < last ) {
-         m.ptr = __ldg( T.bptr + q );
-         m.width = __ldg( T.bptr + q + 1 );
-         m.row = __ldg( T.row + 32 * (int64_t) q + lane );
-         m.len = __ldg( T.len + 32 * (int64_t) q + lane );
+      Meta m{ -1, 0, 0, 0, 0, Real( 1 ) };
+      if( FULL ? q < last : lane < head.z ) {
+         const int at = FULL ? 32 * q + lane : head.x + lane;
+         m.row = __ldg( T.row + at );
+         m.len = __ldg( T.len + at );
          if( UPPER )
-            m.dg = __ldg( T.dg + 32 * (int64_t) q + lane );
+            m.dg = __ldg( T.dg + at );
       }
+      const int4 h = FULL ? load_head( q ) : head;
+      m.slot = h.y + lane;
+      m.rows = FULL ? 32 : h.z;
+      m.width = h.w;
       return m;
    };
    auto load_slots = [ & ]( const Meta& m, int k0, Slots& s )
    {
-      const int64_t g = 32 * (int64_t) ( m.ptr + k0 ) + lane;
+      const int step = FULL ? 32 : m.rows, g = m.slot + k0 * step;
 #pragma unroll
       for( int k = 0; k < kTrsvSlots; k++ ) {
          s.col[ k ] = c0;  // no element: a place of this block
          s.val[ k ] = 0;
          if( k0 + k < m.len ) {
-            s.col[ k ] = __ldg( T.col + g + 32 * k );
-            s.val[ k ] = __ldg( T.val + g + 32 * k );
+            s.col[ k ] = __ldg( T.col + g + k * step );
+            s.val[ k ] = __ldg( T.val + g + k * step );
          }
       }
    };
    int q = T.bfirst[ blk ] + warp;
-   Meta next = load_meta( q ), after = load_meta( q + kTrsvWarps );
+   const int4 none = make_int4( 0, 0, 0, 0 );
+   Meta next = load_meta( q, FULL ? none : load_head( q ) );
+   Meta after = load_meta( q + kTrsvWarps, FULL ? none : load_head( q + kTrsvWarps ) );
+   int4 head = FULL ? none : load_head( q + 2 * kTrsvWarps );
    Slots ahead;
    auto load_ahead = [ & ]()
    {
@@ -453,7 +464,6 @@ ilu_block_trsv_kernel( TrsvView< Real > T, IluState* st, const Real* b, typename
    for( ; q < last; q += kTrsvWarps ) {
       const Meta m = next;
       Slots s = ahead;
-      const int width = m.width - m.ptr;
       Real acc = s.b;
       // where the slots' values are: in xs, or (at < 0) in another block's,
       // whose first look goes out now
@@ -474,8 +484,10 @@ ilu_block_trsv_kernel( TrsvView< Real > T, IluState* st, const Real* b, typename
       look( 0 );
       next = after;
       load_ahead();
-      after = load_meta( q + 2 * kTrsvWarps );
-      for( int k0 = 0; k0 < width; k0 += kTrsvSlots ) {
+      after = load_meta( q + 2 * kTrsvWarps, head );
+      if( ! FULL )
+         head = load_head( q + 3 * kTrsvWarps );
+      for( int k0 = 0; k0 < m.width; k0 += kTrsvSlots ) {
          if( k0 > 0 ) {
             load_slots( m, k0, s );
             look( k0 );
@@ -539,32 +551,38 @@ ilu_block_trsv_kernel( TrsvView< Real > T, IluState* st, const Real* b, typename
       atomicExch( &st->error, 1 );
 }
 
-// the packed rows of one triangle (slots, lengths, diagonal) from the factors
+// the packed rows of one triangle (slots, lengths, diagonal) from the factors,
+// a warp per batch
 template< typename Real, bool UPPER >
 __global__ void
-trsv_pack_kernel( int32_t lanes, const int32_t* __restrict__ row, const int32_t* __restrict__ bptr,
+trsv_pack_kernel( int32_t batches, const int4* __restrict__ batch, const int32_t* __restrict__ row,
                   const int32_t* __restrict__ off, const int32_t* __restrict__ diag, const int32_t* __restrict__ col,
                   const Real* __restrict__ lu, int32_t* __restrict__ len, int32_t* __restrict__ pcol,
                   Real* __restrict__ pval, Real* __restrict__ dg )
 {
+   const int64_t lanes = 32 * (int64_t) batches;
    for( int64_t t = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; t < lanes; t += (int64_t) gridDim.x * blockDim.x ) {
-      const int i = row[ t ];
+      const int4 h = batch[ t >> 5 ];
+      const int l = (int) ( t & 31 );
+      if( l >= h.z )
+         continue;
+      const int i = row[ h.x + l ];
       if( i < 0 ) {
-         len[ t ] = 0;
+         len[ h.x + l ] = 0;
          if( UPPER )
-            dg[ t ] = 1;
+            dg[ h.x + l ] = 1;
          continue;
       }
       const int d = diag[ i ];
       const int b0 = UPPER ? d + 1 : off[ i ], b1 = UPPER ? off[ i + 1 ] : d;
-      const int64_t g = 32 * (int64_t) bptr[ t >> 5 ] + ( t & 31 );
+      const int g = h.y + l;
       for( int k = b0; k < b1; k++ ) {
-         pcol[ g + 32 * (int64_t) ( k - b0 ) ] = col[ k ];
-         pval[ g + 32 * (int64_t) ( k - b0 ) ] = lu[ k ];
+         pcol[ g + ( k - b0 ) * h.z ] = col[ k ];
+         pval[ g + ( k - b0 ) * h.z ] = lu[ k ];
       }
-      len[ t ] = b1 - b0;
+      len[ h.x + l ] = b1 - b0;
       if( UPPER )
-         dg[ t ] = lu[ d ];
+         dg[ h.x + l ] = lu[ d ];
    }
 }
 
@@ -580,15 +598,16 @@ trsv_clear_kernel( Bits* y, int64_t count, Bits v )
 template< typename Real >
 struct TrsvPlan
 {
-   DevBuf bfirst, bptr, row, len, col, val, dg;
+   DevBuf bfirst, batch, row, len, col, val, dg;
    int32_t batches = 0;
+   bool full = false;  // 32 lanes to every batch
 
    TrsvView< Real > view( int32_t n, int32_t rows_per_block ) const
    {
       return TrsvView< Real >{ n,
                                rows_per_block,
                                bfirst.as< int32_t >(),
-                               bptr.as< int32_t >(),
+                               batch.as< int4 >(),
                                row.as< int32_t >(),
                                len.as< int32_t >(),
                                col.as< int32_t >(),
@@ -650,12 +669,21 @@ struct IluFactors
       using Bits = typename TrsvBits< Real >::type;
       Bits *y = yz.as< Bits >(), *z = y + n;
       const size_t smem = (size_t) rows_per_block * sizeof( Real );
-      B2S_TRY( allow_smem( reinterpret_cast< const void* >( ilu_block_trsv_kernel< Real, false, PLAIN, Gate > ), smem ) );
-      B2S_TRY( allow_smem( reinterpret_cast< const void* >( ilu_block_trsv_kernel< Real, true, PLAIN, Gate > ), smem ) );
-      ilu_block_trsv_kernel< Real, false, PLAIN, Gate >
-         <<< blocks, kTrsvBlock, smem, s >>>( plan_l.view( n, rows_per_block ), state.as< IluState >(), b, y, z, x, gate );
-      ilu_block_trsv_kernel< Real, true, PLAIN, Gate ><<< blocks, kTrsvBlock, smem, s >>>(
-         plan_u.view( n, rows_per_block ), state.as< IluState >(), reinterpret_cast< const Real* >( y ), z, y, x, gate );
+      const Real* yr = reinterpret_cast< const Real* >( y );
+      B2S_TRY( ( plan_l.full ? pass< false, PLAIN, true >( plan_l, b, y, z, x, smem, s, gate )
+                             : pass< false, PLAIN, false >( plan_l, b, y, z, x, smem, s, gate ) ) );
+      return plan_u.full ? pass< true, PLAIN, true >( plan_u, yr, z, y, x, smem, s, gate )
+                         : pass< true, PLAIN, false >( plan_u, yr, z, y, x, smem, s, gate );
+   }
+
+   template< bool UPPER, bool PLAIN, bool FULL, class Bits, class Gate >
+   b2s_status pass( const TrsvPlan< Real >& P, const Real* b, Bits* pub, Bits* other, Real* x, size_t smem, cudaStream_t s,
+                    Gate gate ) const
+   {
+      auto kern = ilu_block_trsv_kernel< Real, UPPER, PLAIN, FULL, Gate >;
+      B2S_TRY( allow_smem( reinterpret_cast< const void* >( kern ), smem ) );
+      kern<<< blocks, kTrsvBlock, smem, s >>>( P.view( n, rows_per_block ), state.as< IluState >(), b, pub, other, x,
+                                               gate );
       B2S_TRY_CUDA( cudaGetLastError() );
       return B2S_OK;
    }
