@@ -512,6 +512,12 @@ typedef struct
 b2s_status b2s_solver_create( b2s_matrix A, const b2s_solve_opts* opts, b2s_solver* out );
 b2s_status b2s_solver_destroy( b2s_solver s );
 
+/* Kernels in which blocks wait for one another bound every wait: after `looks`
+ * polls without success it gives up. 0 (the default): the kernels' own limits,
+ * about a second and more. CG and BiCGStab solves go on without such a kernel
+ * when a wait of theirs gave up. TNL has no counterpart. */
+b2s_status b2s_solver_set_wait_limit( b2s_solver s, int32_t looks );
+
 /* bool solve( ConstVectorViewType b, VectorViewType x ) (Solvers/Linear/LinearSolver.h:155-156):
  * x is the initial guess on entry and the solution on exit. Returns B2S_OK when
  * converged, B2S_NOT_CONVERGED / B2S_NAN / B2S_DIVERGED as TNL's solve()

@@ -819,6 +819,8 @@ struct b2s_solver_t
    // exchange slots of the resident CG / BiCGStab kernel (empty: the graph of
    // kernels runs)
    DevBuf resident;
+   bool resident_off = false;  // a wait of that kernel ran out in this solve: the graph takes over
+   int32_t looks = 0;          // polls after which a wait between blocks gives up (0: the kernels' own limits)
 
    // GMRES
    DevBuf gm;
@@ -1069,7 +1071,8 @@ normb_launch( b2s_solver_t* S, const Real* b, const Real* diag )
 
 // Iterations of the resident kernel until it says done or stops early: it
 // runs at most `kResidentIterations` per launch, so that other streams get
-// their turn and the wall clock is looked at.
+// their turn and the wall clock is looked at. Returns with resident_off set,
+// and the state of before the last launch, when a wait ran out.
 constexpr int kResidentIterations = 1000;
 
 template< typename Real >
@@ -1078,15 +1081,22 @@ resident_run( b2s_solver_t* S, const Real* vals, const Real* diag, double eps2 )
 {
    auto v = vec_layout< Real >( S );
    Ctl* ctl = S->ctl_buf.as< Ctl >();
-   const ResidentVecs< Real > rv{ v.x, v.r, v.p, v.Ap, v.z, v.r_ast, v.s, v.As };
+   // CG has no r_ast and BiCGStab no z
+   const ResidentVecs< Real > rv{ v.x, v.r, v.p, v.Ap, v.z, v.r_ast, v.s, v.As, v.w, S->o.solver == B2S_CG ? v.r_ast : v.z };
    const int iterations = S->o.check_interval > 0 ? S->o.check_interval : kResidentIterations;
    for( ;; ) {
-      B2S_TRY( resident_iterate< Real >( S->A, S->o.solver, vals, diag, rv, ctl, S->resident, iterations, eps2, S->cs ) );
+      B2S_TRY( resident_iterate< Real >( S->A, S->o.solver, vals, diag, rv, ctl, S->resident, iterations, S->looks, eps2,
+                                         S->cs ) );
       B2S_TRY( read_ctl( S ) );
       if( S->h_ctl->gave_up ) {
+         const size_t bytes = (size_t) S->n * sizeof( Real );
          B2S_TRY( resident_scratch_init( S->resident, S->cs ) );
-         set_error( "solver: a bounded wait between blocks gave up" );
-         return B2S_TIMEOUT;
+         B2S_TRY_CUDA( cudaMemcpyAsync( rv.r, rv.r0, bytes, cudaMemcpyDeviceToDevice, S->cs ) );
+         B2S_TRY_CUDA( cudaMemcpyAsync( rv.p, rv.p0, bytes, cudaMemcpyDeviceToDevice, S->cs ) );
+         B2S_TRY_CUDA( cudaMemsetAsync( &ctl->gave_up, 0, sizeof( int ), S->cs ) );
+         S->h_ctl->gave_up = 0;
+         S->resident_off = true;
+         return B2S_OK;
       }
       if( S->h_ctl->done || S->h_ctl->restart_flag )
          return B2S_OK;
@@ -1139,8 +1149,11 @@ cg_iterate( b2s_solver_t* S, const Real* vals, const Real* diag, long long tagba
    auto v = vec_layout< Real >( S );
    Ctl* ctl = S->ctl_buf.as< Ctl >();
    const IluFactors< Real >* ilu = ilu_of< Real >( S );
-   if( S->resident.p )
-      return resident_run< Real >( S, vals, diag, 0.0 );
+   if( S->resident.p && ! S->resident_off ) {
+      B2S_TRY( resident_run< Real >( S, vals, diag, 0.0 ) );
+      if( ! S->resident_off )
+         return B2S_OK;
+   }
    const int chunk = chunk_of( S );
    for( ;; ) {
       B2S_TRY( run_graph( S, tagbase + chunk, [ & ]() -> b2s_status
@@ -1242,8 +1255,10 @@ bicgstab_iterate( b2s_solver_t* S, const Real* vals, const Real* diag, long long
       s.exact = exact;
       return s;
    };
-   while( S->resident.p ) {
+   while( S->resident.p && ! S->resident_off ) {
       B2S_TRY( resident_run< Real >( S, vals, diag, eps * eps ) );
+      if( S->resident_off )
+         break;
       if( S->h_ctl->done )
          return B2S_OK;
       // r became too orthogonal to r_ast: a new r0, the next direction, and on
@@ -2757,6 +2772,15 @@ b2s_solver_create( b2s_matrix A, const b2s_solve_opts* opts, b2s_solver* out )
 }
 
 b2s_status
+b2s_solver_set_wait_limit( b2s_solver S, int32_t looks )
+{
+   clear_error();
+   B2S_CHECK_ARG( S && looks >= 0, "solver handle / looks" );
+   S->looks = looks;
+   return B2S_OK;
+}
+
+b2s_status
 b2s_solver_destroy( b2s_solver s )
 {
    clear_error();
@@ -2776,6 +2800,7 @@ b2s_solve( b2s_solver S, const void* b, void* x, b2s_memory where, b2s_stream st
    const int64_t n = S->n;
    cudaStream_t us = as_stream( stream );
    S->t_start = std::chrono::steady_clock::now();
+   S->resident_off = false;
    if( S->generation != S->A->generation ) {
       S->drop_graphs();
       if( S->o.solver == B2S_SOR )  // the sweep's plan points into A

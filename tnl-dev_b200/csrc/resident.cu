@@ -20,8 +20,11 @@
 //     direction and s updates need no meeting of their own: two meetings per
 //     CG iteration, three per BiCGStab iteration. Every element is the same
 //     expression wherever it is formed, so results do not depend on it.
-// Every wait is bounded: after kMeetSpin polls a block raises the error word
-// and leaves, as do the others when they see it.
+// Every wait is bounded: after kMeetSpin polls a block marks the count and
+// leaves, as do the others when they see the mark. The mark is set only while
+// the count is short of the meeting, so at the last meeting either every block
+// goes on and writes its part of the result or none does, and the host goes
+// on from the state before the launch with the graph of kernels.
 // Measured per iteration, graph of kernels before: CG in FP64 32^2 11.5 -> 3.4
 // us, 256^2 12.2 -> 7.1 us, 500^2 18.4 -> 12.7 us; BiCGStab 10^3 19.7 -> 7.8 us.
 #include "resident.cuh"
@@ -40,7 +43,8 @@ constexpr int kResMaxRows = 8 * kResBlock;
 constexpr int kResMaxRowsBicg64 = 4 * kResBlock;
 constexpr int kResMaxBlocks = 256;             // slots per set and value
 constexpr int kResSmemMax = 200 * 1024;
-constexpr int kMeetSpin = 1 << 22;             // polls of L2, about 2 s
+constexpr int kMeetSpin = 1 << 22;             // polls of L2, 290 cycles or more each: 0.6 s or more
+constexpr unsigned long long kMeetOff = 1ull << 63;  // in the count: a block gave up
 constexpr int kClusterBlocks = 8;
 // Rows up to which one cluster takes the system, four to a thread of its eight
 // blocks (CG, 1,024 rows: 3.4 us per iteration)
@@ -52,10 +56,8 @@ constexpr int kResMinRows = 256;
 struct MeetSlots
 {
    double v[ 2 ][ 2 ][ kResMaxBlocks ];  // [meeting's parity][value][block]
-   unsigned count;                       // blocks counted in, over all meetings of all launches
-   unsigned base;                        // `count` before this launch
-   int error;
-   int pad[ 13 ];
+   unsigned long long count;             // blocks counted in, over all meetings of all launches
+   unsigned long long base;              // `count` before this launch
 };
 
 __device__ __forceinline__ void
@@ -102,7 +104,7 @@ struct ResidentArgs
    ResidentVecs< Real > v;
    Ctl* ctl;
    MeetSlots* slots;
-   int iterations;
+   int iterations, looks;
    double eps2;
 };
 
@@ -114,7 +116,7 @@ struct ResidentArgs
 // all 16 warps takes longer than in one).
 template< int NV, bool CLUSTER, class Fin >
 __device__ __forceinline__ bool
-meet( double ( &v )[ NV ], MeetSlots* S, unsigned& meeting, unsigned base, Fin&& fin )
+meet( double ( &v )[ NV ], MeetSlots* S, int looks, unsigned& meeting, unsigned long long base, Fin&& fin )
 {
    __shared__ double sh[ NV ][ kResBlock / 32 ];
    __shared__ double part[ 2 ][ NV ];
@@ -154,13 +156,15 @@ meet( double ( &v )[ NV ], MeetSlots* S, unsigned& meeting, unsigned base, Fin&&
          for( int k = 0; k < NV; k++ )
             S->v[ set ][ k ][ blockIdx.x ] = v[ k ];
          meet_fence();
-         atomicAdd( &S->count, 1u );
-         const unsigned want = base + meeting * (unsigned) G;
-         int it = 0;
-         while( (int) ( *(volatile unsigned*) &S->count - want ) < 0 && ok ) {
-            if( ( ++it & 255 ) == 0 && ( it >= kMeetSpin || *(volatile int*) &S->error ) )
-               ok = false;
-         }
+         atomicAdd( &S->count, 1ull );
+         const unsigned long long want = base + (unsigned long long) meeting * (unsigned) G;
+         unsigned long long c;
+         for( int it = 0; ( c = *(volatile unsigned long long*) &S->count ) < want; it++ )
+            if( it >= looks && atomicCAS( &S->count, c, c | kMeetOff ) == c ) {
+               c |= kMeetOff;
+               break;
+            }
+         ok = ( c & kMeetOff ) == 0;
          meet_fence();  // what the others wrote before they counted in is read after this
          gave_up = ok ? 0 : 1;
       }
@@ -179,8 +183,6 @@ meet( double ( &v )[ NV ], MeetSlots* S, unsigned& meeting, unsigned base, Fin&&
    if( tid == 0 )
       fin( v );
    __syncthreads();
-   if( ! ok && tid == 0 )
-      S->error = 1;
    return ok;
 }
 
@@ -253,6 +255,10 @@ resident_kernel( ResidentArgs< Real > a )
       Ap[ j ] = 0;
       d[ j ] = own && a.diag ? a.diag[ i ] : Real( 1 );
       len[ j ] = own ? slen[ t ] : 0;
+      if( ! CLUSTER && own ) {
+         a.v.r0[ i ] = r[ j ];
+         a.v.p0[ i ] = p[ j ];
+      }
    }
    // the iterations' scalars, the same in every block
    __shared__ Ctl c;
@@ -263,11 +269,11 @@ resident_kernel( ResidentArgs< Real > a )
          a.ctl->gave_up = 1;
    };
    unsigned meeting = 0;
-   const unsigned base = *(volatile unsigned*) &a.slots->base;
+   const unsigned long long base = *(volatile unsigned long long*) &a.slots->base;
    // every block's start (its copy of ctl included) precedes any end
    {
       double one[ 1 ] = { 0.0 };
-      if( ! meet< 1, CLUSTER >( one, a.slots, meeting, base, []( const double* ) {} ) )
+      if( ! meet< 1, CLUSTER >( one, a.slots, a.looks, meeting, base, []( const double* ) {} ) )
          return give_up();
    }
    Real *pa = a.v.p, *pb = a.v.p2;      // p of the last direction, and the one being formed
@@ -295,7 +301,7 @@ resident_kernel( ResidentArgs< Real > a )
             Ap[ j ] = s;
             acc[ 0 ] += (double) s * (double) p[ j ];
          }
-         if( ! meet< 1, CLUSTER >( acc, a.slots, meeting, base, [ & ]( const double* t ) {
+         if( ! meet< 1, CLUSTER >( acc, a.slots, a.looks, meeting, base, [ & ]( const double* t ) {
                 // CgApSink::finish
                 c.s2 = t[ 0 ];
                 if( c.s2 == 0.0 ) {
@@ -334,7 +340,7 @@ resident_kernel( ResidentArgs< Real > a )
             }
             acc[ 0 ] += (double) r[ j ] * (double) zz[ j ];
          }
-         if( ! meet< 1, CLUSTER >( acc, a.slots, meeting, base, [ & ]( const double* t ) { CgUpdateFin{}( c, t ); } ) )
+         if( ! meet< 1, CLUSTER >( acc, a.slots, a.looks, meeting, base, [ & ]( const double* t ) { CgUpdateFin{}( c, t ); } ) )
             return give_up();
          live = ! c.done;
          if( live ) {
@@ -368,7 +374,7 @@ resident_kernel( ResidentArgs< Real > a )
             acc[ 0 ] += (double) s * (double) __ldg( a.v.r_ast + i );
          }
          double a1[ 1 ] = { acc[ 0 ] };
-         if( ! meet< 1, CLUSTER >( a1, a.slots, meeting, base,
+         if( ! meet< 1, CLUSTER >( a1, a.slots, a.looks, meeting, base,
                                    [ & ]( const double* t ) { c.bi_alpha = c.rho / t[ 0 ]; } ) )
             return give_up();
          if( ! first ) {
@@ -401,7 +407,7 @@ resident_kernel( ResidentArgs< Real > a )
             acc[ 0 ] += (double) s * (double) s_[ j ];
             acc[ 1 ] += (double) s * (double) s;
          }
-         if( ! meet< 2, CLUSTER >( acc, a.slots, meeting, base,
+         if( ! meet< 2, CLUSTER >( acc, a.slots, a.looks, meeting, base,
                                    [ & ]( const double* t ) { c.omega = t[ 0 ] / t[ 1 ]; } ) )
             return give_up();
          const Real omega = (Real) c.omega;
@@ -417,7 +423,7 @@ resident_kernel( ResidentArgs< Real > a )
             acc[ 0 ] += (double) r[ j ] * (double) __ldg( a.v.r_ast + i );
             acc[ 1 ] += (double) r[ j ] * (double) r[ j ];
          }
-         if( ! meet< 2, CLUSTER >( acc, a.slots, meeting, base, [ & ]( const double* t ) { BiXrFin{ a.eps2, 0 }( c, t ); } ) )
+         if( ! meet< 2, CLUSTER >( acc, a.slots, a.looks, meeting, base, [ & ]( const double* t ) { BiXrFin{ a.eps2, 0 }( c, t ); } ) )
             return give_up();
          if( c.restart_flag )
             break;
@@ -433,7 +439,7 @@ resident_kernel( ResidentArgs< Real > a )
    // every block has left the gathers of its last direction: the vectors may be put back
    {
       double one[ 1 ] = { 0.0 };
-      if( ! meet< 1, CLUSTER >( one, a.slots, meeting, base, []( const double* ) {} ) )
+      if( ! meet< 1, CLUSTER >( one, a.slots, a.looks, meeting, base, []( const double* ) {} ) )
          return give_up();
    }
 #pragma unroll
@@ -467,7 +473,7 @@ resident_kernel( ResidentArgs< Real > a )
          o.alpha = c.alpha;
          o.beta = c.beta;
       }
-      a.slots->base = base + meeting * gridDim.x;
+      a.slots->base = base + (unsigned long long) meeting * gridDim.x;
    }
    if constexpr( CLUSTER )
       cooperative_groups::this_cluster().sync();  // the others may still read this block's sums
@@ -518,7 +524,6 @@ slots_clear_kernel( MeetSlots* S )
 {
    S->count = 0;
    S->base = 0;
-   S->error = 0;
 }
 
 b2s_status
@@ -581,7 +586,7 @@ launch_resident_rows( const ResidentArgs< Real >& a, int blocks, cudaStream_t s 
 template< typename Real >
 b2s_status
 resident_iterate( const b2s_matrix_t* A, int solver, const Real* vals, const Real* diag, const ResidentVecs< Real >& v,
-                  Ctl* ctl, DevBuf& scratch, int iterations, double eps2, cudaStream_t s )
+                  Ctl* ctl, DevBuf& scratch, int iterations, int looks, double eps2, cudaStream_t s )
 {
    ResidentArgs< Real > a{};
    a.n = A->rows;
@@ -605,6 +610,7 @@ resident_iterate( const b2s_matrix_t* A, int solver, const Real* vals, const Rea
    a.ctl = ctl;
    a.slots = scratch.as< MeetSlots >();
    a.iterations = iterations;
+   a.looks = looks > 0 ? looks : kMeetSpin;
    a.eps2 = eps2;
    if( solver == B2S_BICGSTAB )
       return shape.cluster ? launch_resident_rows< Real, true, true >( a, shape.blocks, s )
@@ -614,8 +620,10 @@ resident_iterate( const b2s_matrix_t* A, int solver, const Real* vals, const Rea
 }
 
 template b2s_status resident_iterate< double >( const b2s_matrix_t*, int, const double*, const double*,
-                                                const ResidentVecs< double >&, Ctl*, DevBuf&, int, double, cudaStream_t );
+                                                const ResidentVecs< double >&, Ctl*, DevBuf&, int, int, double,
+                                                cudaStream_t );
 template b2s_status resident_iterate< float >( const b2s_matrix_t*, int, const float*, const float*,
-                                               const ResidentVecs< float >&, Ctl*, DevBuf&, int, double, cudaStream_t );
+                                               const ResidentVecs< float >&, Ctl*, DevBuf&, int, int, double,
+                                               cudaStream_t );
 
 }  // namespace b2s
