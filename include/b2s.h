@@ -444,6 +444,8 @@ b2s_status b2s_precond_create( b2s_matrix A, int32_t kind, b2s_stream stream, b2
 b2s_status b2s_precond_create_ilut( b2s_matrix A, int32_t p, double threshold, b2s_stream stream, b2s_precond* out );
 b2s_status b2s_precond_solve( b2s_precond M, const void* b, void* x, b2s_memory where, b2s_stream stream );
 b2s_status b2s_precond_destroy( b2s_precond M );
+/* As b2s_solver_set_wait_limit, for the substitutions (B2S_TIMEOUT when a wait gave up). */
+b2s_status b2s_precond_set_wait_limit( b2s_precond M, int32_t looks );
 
 typedef enum
 {

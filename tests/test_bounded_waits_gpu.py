@@ -88,3 +88,52 @@ def test_solves_beside_a_long_kernel(b2s_lib, cuda, kind):
     t.join()
     assert ok == [True] * 3
     assert cuda.equal(alone, mixed)
+
+
+def _chain(n):
+    i = np.repeat(np.arange(n, dtype=np.int64), 3).reshape(n, 3) + np.array([-1, 0, 1])
+    keep = (i >= 0) & (i < n)
+    off = np.concatenate([[0], np.cumsum(keep.sum(axis=1))]).astype(np.int32)
+    val = np.random.default_rng(3).uniform(-1, 1, i.shape)
+    val[:, 1] = 4.0
+    return off, i[keep].astype(np.int32), val[keep], n
+
+
+def test_substitutions_give_up_and_recover(b2s_lib, cuda, oracle):
+    csr = _chain(20000)  # three blocks
+    n = csr[3]
+    M = b2s_lib.SparseMatrix.from_csr(*csr[:3], n)
+    b = np.random.default_rng(4).uniform(-1, 1, n)
+    want = oracle.ilu0_apply(csr, b, "f64")
+    P = b2s_lib.Preconditioner(M, "ilu0")
+    bd = cuda.tensor(b, device="cuda")
+    x = cuda.zeros_like(bd)
+    for _ in range(2):
+        assert b2s_lib.lib.b2s_precond_set_wait_limit(P._h, 1) == b2s_lib.OK
+        with pytest.raises(b2s_lib.B2SError) as e:
+            P.solve(bd, x)
+        assert "gave up" in str(e.value)
+        assert b2s_lib.lib.b2s_precond_set_wait_limit(P._h, 0) == b2s_lib.OK
+        P.solve(bd, x)
+        assert np.array_equal(x.cpu().numpy(), want)
+    s = _solver(b2s_lib, "BICGStab", M, "ilu0")
+    _limit(b2s_lib, s, 1)
+    with pytest.raises(b2s_lib.B2SError) as e:
+        s.solve(bd, x)
+    assert "gave up" in str(e.value)
+    _limit(b2s_lib, s, 0)
+    x.zero_()
+    assert s.solve(bd, x)
+
+
+def test_substitutions_of_a_long_chain(b2s_lib, cuda):
+    """Millions of dependent steps take longer than a fixed limit: the limits follow the chain."""
+    n = 3_700_000
+    off, col, val, _ = _chain(n)
+    val[:] = np.where(col == np.repeat(np.arange(n), np.diff(off)), 4.0, -1.0)
+    P = b2s_lib.Preconditioner(b2s_lib.SparseMatrix.from_csr(off, col, val, n), "ilu0")
+    b = np.full(n, 2.0)
+    b[[0, -1]] = 3.0  # A times 1, and for a tridiagonal matrix ILU(0) is exact
+    x = cuda.zeros(n, dtype=cuda.float64, device="cuda")
+    P.solve(cuda.tensor(b, device="cuda"), x)
+    assert float((x - 1).abs().max()) <= 1e-14  # dominant by 2: each step halves an error, a few ulp are left

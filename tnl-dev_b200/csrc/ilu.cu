@@ -86,7 +86,8 @@ constexpr int64_t kTrsvFullLanes = 3;
 // up to 32 rows of one level. deps( i ): row i's entries in this triangle.
 template< typename Real, class Deps >
 static b2s_status
-block_plan( IluFactors< Real >& F, TrsvPlan< Real >& P, const std::vector< int32_t >& lev, Deps deps, cudaStream_t s )
+block_plan( IluFactors< Real >& F, TrsvPlan< Real >& P, const std::vector< int32_t >& lev, int depth, Deps deps,
+            cudaStream_t s )
 {
    const int32_t G = F.blocks, R = F.rows_per_block;
    std::vector< int32_t > first( (size_t) G + 1, 0 ), row( (size_t) F.n ), count;
@@ -153,6 +154,15 @@ block_plan( IluFactors< Real >& F, TrsvPlan< Real >& P, const std::vector< int32
       h.y = (int32_t) slots;
       slots += (int64_t) h.z * h.w;
    }
+   // the longest row of each level
+   std::vector< int32_t > longest( (size_t) depth, 0 );
+   for( const int4& h : batch ) {
+      int32_t& w = longest[ lev[ row[ h.x ] ] ];
+      w = std::max( w, h.w );
+   }
+   P.steps = 0;
+   for( const int32_t w : longest )
+      P.steps += 1 + w / kTrsvSlots;
    B2S_TRY( P.bfirst.alloc( first.size() * sizeof( int32_t ) ) );
    B2S_TRY( P.batch.alloc( batch.size() * sizeof( int4 ) ) );
    B2S_TRY( P.row.alloc( row.size() * sizeof( int32_t ) ) );
@@ -230,7 +240,7 @@ ilu_levels( IluFactors< Real >& F, const std::vector< int32_t >& hoff, const std
    F.levels_l = depth;
    B2S_TRY( order( depth, F.ord_l, F.n_ord_l ) );
    if( F.blocks > 0 )
-      B2S_TRY( block_plan< Real >( F, F.plan_l, lev, [ & ]( int32_t i ) { return hdiag[ i ] - hoff[ i ]; }, s ) );
+      B2S_TRY( block_plan< Real >( F, F.plan_l, lev, depth, [ & ]( int32_t i ) { return hdiag[ i ] - hoff[ i ]; }, s ) );
    depth = 0;
    for( int32_t i = n - 1; i >= 0; i-- ) {
       int l = 0;
@@ -241,7 +251,7 @@ ilu_levels( IluFactors< Real >& F, const std::vector< int32_t >& hoff, const std
    }
    F.levels_u = depth;
    if( F.blocks > 0 )
-      B2S_TRY( block_plan< Real >( F, F.plan_u, lev, [ & ]( int32_t i ) { return hoff[ i + 1 ] - hdiag[ i ] - 1; }, s ) );
+      B2S_TRY( block_plan< Real >( F, F.plan_u, lev, depth, [ & ]( int32_t i ) { return hoff[ i + 1 ] - hdiag[ i ] - 1; }, s ) );
    if( F.blocks == 0 ) {
       F.plan_l = TrsvPlan< Real >();  // made before U's rows turned out not to suit
       B2S_TRY( order( depth, F.ord_u, F.n_ord_u ) );  // for the warp-per-row kernel (L's also for the factorization)
@@ -473,6 +483,15 @@ b2s_precond_solve( b2s_precond M, const void* b, void* x, b2s_memory where, b2s_
    B2S_TRY_CUDA( cudaStreamSynchronize( s ) );
    if( M->kind == B2S_PRECOND_ILU0 || M->kind == B2S_PRECOND_ILUT )
       return M->dtype == B2S_F64 ? M->f64.check( s ) : M->f32.check( s );
+   return B2S_OK;
+}
+
+b2s_status
+b2s_precond_set_wait_limit( b2s_precond M, int32_t looks )
+{
+   clear_error();
+   B2S_CHECK_ARG( M && looks >= 0, "preconditioner handle / looks" );
+   M->f64.looks = M->f32.looks = looks;
    return B2S_OK;
 }
 

@@ -292,8 +292,9 @@ ilu_trsv_kernel( IluView< Real > L, const Real* b, Real* x )
 //   * Both passes publish in their own scratch vector (y: L^-1 b, z: U^-1 y);
 //     each pass puts the other's scratch back to the signalling NaN for the
 //     next application, so there is no pass to clear them, and b may be x.
-// Every wait is bounded as above (the limits are longer: a block may wait for
-// all blocks before it). Rows per block: see choose_blocks.
+// Every wait is bounded as above. A block may wait for all blocks before it,
+// so the limits grow with the steps of the chain (TrsvPlan::steps). Rows per
+// block: see choose_blocks.
 // Measured, both substitutions of one application through the public call
 // (warp per row before): 3D stencils 10^3 177 -> 52 us, 32^3 535 -> 132 us,
 // 64^3 1,106 -> 284 us, 128^3 3,748 -> 1,009 us; 2D 140^2 1,233 -> 234 us.
@@ -301,8 +302,11 @@ constexpr int kTrsvBlock = 256;                // 128 to 512 measured alike
 constexpr int kTrsvWarps = kTrsvBlock / 32;
 constexpr int kTrsvSlots = 4;                  // slots of the next batch loaded ahead
 constexpr int kTrsvSmemMax = 200 * 1024;       // x of one block in shared memory
-constexpr int kTrsvSpinLocal = 1 << 26;        // polls of shared memory (a few seconds)
-constexpr int kTrsvSpinRemote = 1 << 23;       // polls of L2 (about 2 s)
+// Polls that a wait makes: of shared memory (30 cycles or more each) and of L2
+// (300 or more), a second or so at least, and for each step of the chain the
+// time of 4,000 cycles; a step of the 128^3 stencil takes 2,500.
+constexpr int kTrsvSpinLocal = 1 << 26, kTrsvSpinLocalStep = 128;
+constexpr int kTrsvSpinRemote = 1 << 23, kTrsvSpinRemoteStep = 16;
 
 template< typename Real >
 struct TrsvBits;
@@ -368,6 +372,7 @@ template< typename Real >
 struct TrsvView
 {
    int32_t n, rows_per_block;
+   int32_t spin_local, spin_remote;
    const int32_t* bfirst;  // first batch of each block (blocks + 1 entries)
    const int4* batch;      // x: place of a batch's first lane, y: its first slot, z: lanes, w: slots per lane
    const int32_t* row;     // rows in batch order (-1: a lane without one)
@@ -406,7 +411,7 @@ ilu_block_trsv_kernel( TrsvView< Real > T, IluState* st, const Real* b, typename
    }
    __syncthreads();
    const int last = T.bfirst[ blk + 1 ];
-   bool ok = true;  // false once a wait gave up: no more waits, the count goes on
+   bool ok = true;  // false once a wait gave up: this lane waits no more
    // a batch's lane: loaded three batches (head; two if FULL), two (meta) and one
    // (slots, right-hand side) ahead of its turn, so that no turn waits for them
    struct Meta
@@ -502,7 +507,7 @@ ilu_block_trsv_kernel( TrsvView< Real > T, IluState* st, const Real* b, typename
          if( have ) {
             some = __shfl_sync( 0xffffffffu, some, __ffs( have ) - 1 );
             for( int it = 0; *(volatile Bits*) &xs[ some ] == pending && ok; it++ )
-               if( ( it & 1023 ) == 1023 && ( it >= kTrsvSpinLocal || *(volatile int*) &st->error ) )
+               if( ( it & 1023 ) == 1023 && ( it >= T.spin_local || *(volatile int*) &st->error ) ) 
                   ok = false;
          }
          // The step's latency is what counts from here to the store of x: no
@@ -523,7 +528,7 @@ ilu_block_trsv_kernel( TrsvView< Real > T, IluState* st, const Real* b, typename
                xv[ k ] = at[ k ] < 0 ? xr[ k ] : xv[ k ];
                wait = wait || xv[ k ] == pending;
             }
-            if( ( ++it & 255 ) == 0 && ( it >= kTrsvSpinRemote || *(volatile int*) &st->error ) )
+            if( ( ++it & 255 ) == 0 && ( it >= T.spin_remote || *(volatile int*) &st->error ) ) 
                ok = false;
          } while( __any_sync( 0xffffffffu, wait && ok ) );
 #pragma unroll
@@ -601,11 +606,20 @@ struct TrsvPlan
    DevBuf bfirst, batch, row, len, col, val, dg;
    int32_t batches = 0;
    bool full = false;  // 32 lanes to every batch
+   int64_t steps = 0;  // of the chain: over the levels, the longest row's in groups of kTrsvSlots
 
-   TrsvView< Real > view( int32_t n, int32_t rows_per_block ) const
+   static int32_t limit( int64_t base, int64_t per_step, int64_t steps )
+   {
+      return (int32_t) std::min< int64_t >( base + per_step * steps, 1 << 30 );
+   }
+
+   // looks: the polls after which a wait gives up (0: by the chain's length)
+   TrsvView< Real > view( int32_t n, int32_t rows_per_block, int32_t looks ) const
    {
       return TrsvView< Real >{ n,
                                rows_per_block,
+                               looks > 0 ? looks : limit( kTrsvSpinLocal, kTrsvSpinLocalStep, steps ),
+                               looks > 0 ? looks : limit( kTrsvSpinRemote, kTrsvSpinRemoteStep, steps ),
                                bfirst.as< int32_t >(),
                                batch.as< int4 >(),
                                row.as< int32_t >(),
@@ -633,6 +647,7 @@ struct IluFactors
    TrsvPlan< Real > plan_l, plan_u;
    DevBuf yz;  // the two passes' scratch vectors
    int32_t blocks = 0, rows_per_block = 0;
+   int32_t looks = 0;  // polls after which a wait of theirs gives up (0: by the chain's length)
 
    IluView< Real > view() const
    {
@@ -682,7 +697,7 @@ struct IluFactors
    {
       auto kern = ilu_block_trsv_kernel< Real, UPPER, PLAIN, FULL, Gate >;
       B2S_TRY( allow_smem( reinterpret_cast< const void* >( kern ), smem ) );
-      kern<<< blocks, kTrsvBlock, smem, s >>>( P.view( n, rows_per_block ), state.as< IluState >(), b, pub, other, x,
+      kern<<< blocks, kTrsvBlock, smem, s >>>( P.view( n, rows_per_block, looks ), state.as< IluState >(), b, pub, other, x,
                                                gate );
       B2S_TRY_CUDA( cudaGetLastError() );
       return B2S_OK;

@@ -2777,6 +2777,8 @@ b2s_solver_set_wait_limit( b2s_solver S, int32_t looks )
    clear_error();
    B2S_CHECK_ARG( S && looks >= 0, "solver handle / looks" );
    S->looks = looks;
+   S->ilu64.looks = S->ilu32.looks = looks;
+   S->drop_graphs();  // the substitutions were captured with their limits
    return B2S_OK;
 }
 
