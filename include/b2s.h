@@ -519,6 +519,9 @@ b2s_status b2s_solver_destroy( b2s_solver s );
  * about a second and more. CG and BiCGStab solves go on without such a kernel
  * when a wait of theirs gave up. TNL has no counterpart. */
 b2s_status b2s_solver_set_wait_limit( b2s_solver s, int32_t looks );
+/* A solve that has not ended `seconds` after its call returns B2S_TIMEOUT; looked
+ * at between launches. 0 (the default): 1,800. */
+b2s_status b2s_solver_set_time_limit( b2s_solver s, double seconds );
 
 /* bool solve( ConstVectorViewType b, VectorViewType x ) (Solvers/Linear/LinearSolver.h:155-156):
  * x is the initial guess on entry and the solution on exit. Returns B2S_OK when

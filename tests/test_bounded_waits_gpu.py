@@ -137,3 +137,27 @@ def test_substitutions_of_a_long_chain(b2s_lib, cuda):
     x = cuda.zeros(n, dtype=cuda.float64, device="cuda")
     P.solve(cuda.tensor(b, device="cuda"), x)
     assert float((x - 1).abs().max()) <= 1e-14  # dominant by 2: each step halves an error, a few ulp are left
+
+
+@pytest.mark.parametrize("n", [5, 3001, 20001])  # one block, one cluster, all blocks
+@pytest.mark.parametrize("mixed", [False, True])
+def test_bicgstab_restarts_within_the_time_limit(b2s_lib, cuda, n, mixed):
+    """4 I + a cyclic shift, b = e_0: after the first step r is orthogonal to r_ast exactly, so
+    BiCGStab restarts. Restarts count no iteration: only the clock ends a solve of nothing else."""
+    off = np.arange(0, 2 * n + 1, 2, dtype=np.int32)
+    col = np.sort(np.stack([np.arange(n), (np.arange(n) - 1) % n], axis=1), axis=1).astype(np.int32)
+    val = np.where(col == np.arange(n)[:, None], 4.0, 1.0)
+    M = b2s_lib.SparseMatrix.from_csr(off, col.reshape(-1), val.reshape(-1), n, keep_fp32_copy=mixed)
+    s = _solver(b2s_lib, "BICGStab", M, mixed=mixed)
+    s._ensure()
+    b = cuda.zeros(n, dtype=cuda.float64, device="cuda")
+    b[0] = 1.0
+    x = cuda.zeros_like(b)
+    assert b2s_lib.lib.b2s_solver_set_time_limit(s._solver, 1e-9) == b2s_lib.OK
+    with pytest.raises(b2s_lib.B2SError) as e:
+        s.solve(b, x)
+    assert "exceeded" in str(e.value)
+    assert b2s_lib.lib.b2s_solver_set_time_limit(s._solver, 0.0) == b2s_lib.OK
+    x.zero_()
+    assert s.solve(b, x)
+    assert float((b - 4.0 * x - cuda.roll(x, 1)).norm()) <= 2e-10

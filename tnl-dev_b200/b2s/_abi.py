@@ -155,6 +155,7 @@ PROTOTYPES = {
     "b2s_solver_create": (_st, [_vp, C.POINTER(SolveOpts), C.POINTER(_vp)]),
     "b2s_solver_destroy": (_st, [_vp]),
     "b2s_precond_set_wait_limit": (_st, [_vp, C.c_int32]),
+    "b2s_solver_set_time_limit": (_st, [_vp, C.c_double]),
     "b2s_solver_set_wait_limit": (_st, [_vp, C.c_int32]),
     "b2s_solve": (_st, [_vp, _vp, _vp, C.c_int, _vp, C.POINTER(SolveReport)]),
     "b2s_scan_i32_noalloc": (_st, [C.c_int64, _vp, C.c_int32, _vp]),

@@ -787,6 +787,13 @@ using namespace b2s;
 
 // ---------------------------------------------------------------------------
 // Solver handle
+namespace b2s {
+// Host-side bound on one solve: the polling loops end with B2S_TIMEOUT
+// instead of running forever if the device never reports completion.
+constexpr double kMaxSolveSeconds = 1800.0;
+
+}  // namespace b2s
+
 struct b2s_solver_t
 {
    b2s_matrix_t* A = nullptr;
@@ -834,6 +841,7 @@ struct b2s_solver_t
    uint64_t generation = 0;
    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
    std::chrono::steady_clock::time_point t_start;
+   double max_seconds = kMaxSolveSeconds;
 
    void drop_graphs()
    {
@@ -966,16 +974,12 @@ run_graph( b2s_solver_t* S, long long key, F&& body )
    return B2S_OK;
 }
 
-// Host-side bound on one solve: the polling loops end with B2S_TIMEOUT
-// instead of running forever if the device never reports completion.
-constexpr double kMaxSolveSeconds = 1800.0;
-
 static b2s_status
 check_wall( b2s_solver_t* S )
 {
    const double s = std::chrono::duration< double >( std::chrono::steady_clock::now() - S->t_start ).count();
-   if( s > kMaxSolveSeconds ) {
-      set_error( "solve exceeded %.0f s without the device reporting completion", kMaxSolveSeconds );
+   if( s > S->max_seconds ) {
+      set_error( "solve exceeded %g s without the device reporting completion", S->max_seconds );
       return B2S_TIMEOUT;
    }
    return B2S_OK;
@@ -1098,9 +1102,11 @@ resident_run( b2s_solver_t* S, const Real* vals, const Real* diag, double eps2 )
          S->resident_off = true;
          return B2S_OK;
       }
-      if( S->h_ctl->done || S->h_ctl->restart_flag )
+      if( S->h_ctl->done )
          return B2S_OK;
-      B2S_TRY( check_wall( S ) );
+      B2S_TRY( check_wall( S ) );  // before a restart too: restarts count no iteration
+      if( S->h_ctl->restart_flag )
+         return B2S_OK;
    }
 }
 
@@ -2779,6 +2785,15 @@ b2s_solver_set_wait_limit( b2s_solver S, int32_t looks )
    S->looks = looks;
    S->ilu64.looks = S->ilu32.looks = looks;
    S->drop_graphs();  // the substitutions were captured with their limits
+   return B2S_OK;
+}
+
+b2s_status
+b2s_solver_set_time_limit( b2s_solver S, double seconds )
+{
+   clear_error();
+   B2S_CHECK_ARG( S && seconds >= 0, "solver handle / seconds" );
+   S->max_seconds = seconds > 0 ? seconds : kMaxSolveSeconds;
    return B2S_OK;
 }
 
