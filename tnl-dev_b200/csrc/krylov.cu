@@ -826,7 +826,8 @@ struct b2s_solver_t
    // exchange slots of the resident CG / BiCGStab kernel (empty: the graph of
    // kernels runs)
    DevBuf resident;
-   bool resident_off = false;  // a wait of that kernel ran out in this solve: the graph takes over
+   int resident_failures = 0;  // waits of that kernel that ran out in this solve
+   bool resident_off = false;  // too many: the graph takes over
    int32_t looks = 0;          // polls after which a wait between blocks gives up (0: the kernels' own limits)
 
    // GMRES
@@ -1075,9 +1076,11 @@ normb_launch( b2s_solver_t* S, const Real* b, const Real* diag )
 
 // Iterations of the resident kernel until it says done or stops early: it
 // runs at most `kResidentIterations` per launch, so that other streams get
-// their turn and the wall clock is looked at. Returns with resident_off set,
-// and the state of before the last launch, when a wait ran out.
+// their turn and the wall clock is looked at. When a wait ran out it is
+// launched again from the state before (the result keeps its bits), and the
+// second time returns with resident_off set and that state.
 constexpr int kResidentIterations = 1000;
+constexpr int kResidentTries = 2;
 
 template< typename Real >
 static b2s_status
@@ -1099,8 +1102,11 @@ resident_run( b2s_solver_t* S, const Real* vals, const Real* diag, double eps2 )
          B2S_TRY_CUDA( cudaMemcpyAsync( rv.p, rv.p0, bytes, cudaMemcpyDeviceToDevice, S->cs ) );
          B2S_TRY_CUDA( cudaMemsetAsync( &ctl->gave_up, 0, sizeof( int ), S->cs ) );
          S->h_ctl->gave_up = 0;
-         S->resident_off = true;
-         return B2S_OK;
+         S->resident_off = ++S->resident_failures >= kResidentTries;
+         if( S->resident_off )
+            return B2S_OK;
+         B2S_TRY( check_wall( S ) );
+         continue;
       }
       if( S->h_ctl->done )
          return B2S_OK;
@@ -2817,6 +2823,7 @@ b2s_solve( b2s_solver S, const void* b, void* x, b2s_memory where, b2s_stream st
    const int64_t n = S->n;
    cudaStream_t us = as_stream( stream );
    S->t_start = std::chrono::steady_clock::now();
+   S->resident_failures = 0;
    S->resident_off = false;
    if( S->generation != S->A->generation ) {
       S->drop_graphs();
