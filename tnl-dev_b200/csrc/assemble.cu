@@ -152,20 +152,45 @@ grid_of( int64_t n, int threads = 256 )
    return (int) std::max< int64_t >( 1, std::min< int64_t >( g, (int64_t) num_sms() * 32 ) );
 }
 
-// Sorts keys[0, n) (with payload idx) stably on their low `bits` bits; the
-// result is in *keys / *idx (the buffers may be swapped with the spares).
+// consecutive pieces of one allocation, each on a 256-byte boundary
+struct Pieces
+{
+   DevBuf buf;
+   size_t used = 0;
+   template< typename T >
+   size_t add( size_t count )
+   {
+      const size_t at = used;
+      used += ( count * sizeof( T ) + 511 ) / 256 * 256;
+      return at;
+   }
+   template< typename T >
+   T* at( size_t offset ) const
+   {
+      return reinterpret_cast< T* >( static_cast< char* >( buf.p ) + offset );
+   }
+};
+
+// keys with their payload, and the spares of a sort
+struct SortSpace
+{
+   uint64_t *keys, *keys2;
+   int32_t *idx, *idx2;
+   int* flag;
+};
+
+// Sorts S.keys[0, n) (with payload S.idx) stably on their low `bits` bits (the
+// arrays may be swapped with the spares).
 static b2s_status
-radix_sort( DevBuf& keys, DevBuf& idx, DevBuf& keys2, DevBuf& idx2, int64_t n, int bits, cudaStream_t s )
+radix_sort( SortSpace& S, int64_t n, int bits, cudaStream_t s )
 {
    if( n <= 1 || bits <= 0 )
       return B2S_OK;
-   DevBuf flag;
-   B2S_TRY( flag.alloc( sizeof( int ) ) );
-   B2S_TRY_CUDA( cudaMemsetAsync( flag.p, 0, sizeof( int ), s ) );
-   sorted_check_kernel<<< grid_of( n ), 256, 0, s >>>( keys.as< uint64_t >(), n, flag.as< int >() );
+   B2S_TRY_CUDA( cudaMemsetAsync( S.flag, 0, sizeof( int ), s ) );
+   sorted_check_kernel<<< grid_of( n ), 256, 0, s >>>( S.keys, n, S.flag );
    B2S_TRY_CUDA( cudaGetLastError() );
    int unsorted = 0;
-   B2S_TRY( copy_d2h( &unsorted, flag.p, sizeof( int ), s ) );
+   B2S_TRY( copy_d2h( &unsorted, S.flag, sizeof( int ), s ) );
    if( ! unsorted )
       return B2S_OK;
    const int64_t nb = ( n + kRadixTile - 1 ) / kRadixTile;
@@ -176,15 +201,14 @@ radix_sort( DevBuf& keys, DevBuf& idx, DevBuf& keys2, DevBuf& idx2, int64_t n, i
    DevBuf counts;
    B2S_TRY( counts.alloc( (size_t) nb * 256 * sizeof( int64_t ) ) );
    for( int shift = 0; shift < bits; shift += 8 ) {
-      radix_hist_kernel<<< (unsigned) nb, kRadixBlock, 0, s >>>( keys.as< uint64_t >(), n, shift, counts.as< int64_t >() );
+      radix_hist_kernel<<< (unsigned) nb, kRadixBlock, 0, s >>>( S.keys, n, shift, counts.as< int64_t >() );
       B2S_TRY_CUDA( cudaGetLastError() );
       B2S_TRY( scan_exclusive_i64( counts.as< int64_t >(), nb * 256, s ) );
-      radix_scatter_kernel<<< (unsigned) nb, kRadixBlock, 0, s >>>( keys.as< uint64_t >(), idx.as< int32_t >(), n, shift,
-                                                                  counts.as< int64_t >(), keys2.as< uint64_t >(),
-                                                                  idx2.as< int32_t >() );
+      radix_scatter_kernel<<< (unsigned) nb, kRadixBlock, 0, s >>>( S.keys, S.idx, n, shift, counts.as< int64_t >(),
+                                                                  S.keys2, S.idx2 );
       B2S_TRY_CUDA( cudaGetLastError() );
-      std::swap( keys, keys2 );
-      std::swap( idx, idx2 );
+      std::swap( S.keys, S.keys2 );
+      std::swap( S.idx, S.idx2 );
    }
    return B2S_OK;
 }
@@ -282,7 +306,11 @@ i64_to_i32_kernel( const int64_t* __restrict__ in, int64_t n, int32_t* __restric
 // triplets (which also ranks a triplet among its row's), scan the counts, put
 // column and position into the row's place, and sort each row by column and
 // position, 32 rows to a warp in shared memory. Matrices with a row of more
-// than kBucketRow triplets take the radix sort.
+// than kBucketRow triplets take the radix sort: the count stops at the first
+// such row, and both ways share one workspace (a second one of this size costs
+// more than the count: 10 M triplets and a row of 100,000, 18.2 ms with the
+// sort alone, 19.7 with a workspace each, 18.5 shared; 40,000 triplets and a
+// row of 10,000, 1.53, 2.13 and 1.51 ms).
 constexpr int kBucketRow = 32;
 constexpr int kBucketWarps = 4;
 constexpr int kBucketBlock = 32 * kBucketWarps;
@@ -301,6 +329,8 @@ coo_count_kernel( int64_t n, const int32_t* __restrict__ ri, const int32_t* __re
 {
    int most = 0;
    for( int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x ) {
+      // what other threads have seen arrives while this triplet is counted
+      const int others = *(volatile int*) &F->longest;
       const int32_t r = ri[ i ], c = ci[ i ];
       if( r < 0 || r >= rows || c < 0 || c >= cols ) {
          F->bad = 1;
@@ -309,6 +339,10 @@ coo_count_kernel( int64_t n, const int32_t* __restrict__ ri, const int32_t* __re
       const int k = (int) atomicAdd( count + r, 1ull );
       rank[ i ] = k;
       most = max( most, k + 1 );
+      if( k == kBucketRow )
+         atomicMax( &F->longest, k + 1 );
+      if( k >= kBucketRow || others > kBucketRow )
+         break;  // the radix sort's: it checks the rest of the indexes
    }
    most = __reduce_max_sync( 0xffffffffu, most );
    if( ( threadIdx.x & 31 ) == 0 && most > *(volatile int*) &F->longest )
@@ -408,25 +442,6 @@ coo_merge_rows_kernel( int32_t rows, const int32_t* __restrict__ caps, const int
    }
 }
 
-// consecutive pieces of one allocation, each on a 256-byte boundary
-struct Pieces
-{
-   DevBuf buf;
-   size_t used = 0;
-   template< typename T >
-   size_t add( size_t count )
-   {
-      const size_t at = used;
-      used += ( count * sizeof( T ) + 511 ) / 256 * 256;
-      return at;
-   }
-   template< typename T >
-   T* at( size_t offset ) const
-   {
-      return reinterpret_cast< T* >( static_cast< char* >( buf.p ) + offset );
-   }
-};
-
 static int
 bits_for( int64_t v )  // bits needed for values in [0, v)
 {
@@ -458,30 +473,64 @@ user_capacities( const int32_t* caps, const int32_t* used, int32_t rows, int64_t
    return copy_d2h( &total, c64.as< int64_t >() + rows, sizeof( int64_t ), s );
 }
 
+// Workspace of an assembly: 24 bytes per triplet, which the radix sort and the
+// assembly by rows take for one or the other, and what the latter needs per row.
+struct AssembleSpace : Pieces
+{
+   size_t p_keys, p_keys2, p_idx, p_idx2, p_flags;
+   size_t p_off, p_unique, p_caps, p_off32, p_used;
+   bool by_rows = false;
+
+   b2s_status
+   init( int64_t n, int32_t rows, bool used_counts, bool want_rows )
+   {
+      const size_t m = (size_t) rows + 1, count = (size_t) std::max< int64_t >( n, 1 );
+      p_keys = add< uint64_t >( count );
+      p_keys2 = add< uint64_t >( count );
+      p_idx = add< int32_t >( count );
+      p_idx2 = add< int32_t >( count );
+      p_flags = add< BucketFlags >( 1 );
+      const size_t sort_only = used;
+      if( want_rows ) {
+         p_off = add< int64_t >( m );
+         p_unique = add< int64_t >( m );
+         p_caps = add< int32_t >( m );
+         p_off32 = add< int32_t >( m );
+         p_used = add< int32_t >( used_counts ? m : 0 );
+         const b2s_status st = buf.alloc( used );
+         by_rows = st == B2S_OK;
+         if( st != B2S_OOM )
+            return st;
+         clear_error();  // the sort alone may fit
+      }
+      return buf.alloc( sort_only );
+   }
+
+   SortSpace sort_space() const
+   {
+      return SortSpace{ at< uint64_t >( p_keys ), at< uint64_t >( p_keys2 ), at< int32_t >( p_idx ), at< int32_t >( p_idx2 ),
+                        at< int >( p_flags ) };
+   }
+};
+
 // The row-bucket assembly; taken = false (and nothing built) when a row is too
 // long for it.
 template< typename Real, typename Tin >
 static b2s_status
 assemble_rows( b2s_format format, b2s_dtype dtype, int32_t rows, int32_t cols, int64_t n, const int32_t* ri,
                const int32_t* ci, const Tin* vals, int add, const int32_t* caps_user, const b2s_matrix_opts& o,
-               cudaStream_t s, b2s_matrix* out, bool& taken )
+               cudaStream_t s, const AssembleSpace& W, b2s_matrix* out, bool& taken )
 {
    taken = false;
-   if( n == 0 || rows == 0 || n > INT32_MAX )
-      return B2S_OK;
    const size_t m = (size_t) rows + 1;
-   Pieces W;
-   const size_t p_off = W.add< int64_t >( m ), p_rank = W.add< int32_t >( n ), p_flags = W.add< BucketFlags >( 1 ),
-                p_keys = W.add< uint64_t >( n ), p_caps = W.add< int32_t >( m ), p_off32 = W.add< int32_t >( m ),
-                p_unique = W.add< int64_t >( m ), p_col = W.add< int32_t >( n ), p_val = W.add< Real >( n ),
-                p_used = W.add< int32_t >( caps_user ? m : 0 );
-   B2S_TRY( W.buf.alloc( W.used ) );
-   int64_t *off = W.at< int64_t >( p_off ), *unique = W.at< int64_t >( p_unique );
-   int32_t *rank = W.at< int32_t >( p_rank ), *caps = W.at< int32_t >( p_caps ), *off32 = W.at< int32_t >( p_off32 ),
-           *ucol = W.at< int32_t >( p_col );
-   uint64_t* keys = W.at< uint64_t >( p_keys );
-   Real* uval = W.at< Real >( p_val );
-   BucketFlags* F = W.at< BucketFlags >( p_flags );
+   int64_t *off = W.at< int64_t >( W.p_off ), *unique = W.at< int64_t >( W.p_unique );
+   int32_t *caps = W.at< int32_t >( W.p_caps ), *off32 = W.at< int32_t >( W.p_off32 );
+   uint64_t* keys = W.at< uint64_t >( W.p_keys );
+   // ranks and columns in the place of the second keys, values in that of the payloads
+   int32_t *rank = W.at< int32_t >( W.p_keys2 ),
+           *ucol = W.at< int32_t >( W.p_keys2 + ( (size_t) n * sizeof( int32_t ) + 255 ) / 256 * 256 );
+   Real* uval = W.at< Real >( W.p_idx );
+   BucketFlags* F = W.at< BucketFlags >( W.p_flags );
    B2S_TRY_CUDA( cudaMemsetAsync( off, 0, m * sizeof( int64_t ), s ) );
    B2S_TRY_CUDA( cudaMemsetAsync( F, 0, sizeof( BucketFlags ), s ) );
    coo_count_kernel<<< grid_of( n ), 256, 0, s >>>( n, ri, ci, rows, cols, reinterpret_cast< unsigned long long* >( off ),
@@ -508,7 +557,7 @@ assemble_rows( b2s_format format, b2s_dtype dtype, int32_t rows, int32_t cols, i
    }
    else {
       if( caps_user ) {
-         int32_t* used = W.at< int32_t >( p_used );
+         int32_t* used = W.at< int32_t >( W.p_used );
          i64_to_i32_kernel<<< grid_of( (int64_t) m ), 256, 0, s >>>( unique, (int64_t) m, used );
          B2S_TRY( user_capacities( caps_user, used, rows, caps_total, s ) );
          caps_used = caps_user;
@@ -530,50 +579,47 @@ assemble( b2s_format format, b2s_dtype dtype, int32_t rows, int32_t cols, int64_
           const int32_t* ci, const Tin* vals, int add, const int32_t* caps_user, const b2s_matrix_opts& o,
           cudaStream_t s, b2s_matrix* out )
 {
-   bool taken = false;
-   B2S_TRY( ( assemble_rows< Real, Tin >( format, dtype, rows, cols, n, ri, ci, vals, add, caps_user, o, s, out, taken ) ) );
-   if( taken )
-      return B2S_OK;
+   AssembleSpace W;
+   B2S_TRY( W.init( n, rows, caps_user != nullptr,
+                    n > 0 && n <= INT32_MAX && n <= (int64_t) kBucketRow * rows ) );  // more: some row is too long
+   if( W.by_rows ) {
+      bool taken = false;
+      B2S_TRY( ( assemble_rows< Real, Tin >( format, dtype, rows, cols, n, ri, ci, vals, add, caps_user, o, s, W, out,
+                                             taken ) ) );
+      if( taken )
+         return B2S_OK;
+   }
+   SortSpace S = W.sort_space();
    const int cbits = bits_for( cols ), rbits = bits_for( rows );
-   DevBuf keys, idx, keys2, idx2, flag;
-   B2S_TRY( keys.alloc( (size_t) std::max< int64_t >( n, 1 ) * sizeof( uint64_t ) ) );
-   B2S_TRY( idx.alloc( (size_t) std::max< int64_t >( n, 1 ) * sizeof( int32_t ) ) );
-   B2S_TRY( flag.alloc( sizeof( int ) ) );
-   B2S_TRY_CUDA( cudaMemsetAsync( flag.p, 0, sizeof( int ), s ) );
+   B2S_TRY_CUDA( cudaMemsetAsync( S.flag, 0, sizeof( int ), s ) );
    if( n > 0 ) {
-      coo_keys_kernel<<< grid_of( n ), 256, 0, s >>>( n, ri, ci, rows, cols, cbits, keys.as< uint64_t >(),
-                                                      idx.as< int32_t >(), flag.as< int >() );
+      coo_keys_kernel<<< grid_of( n ), 256, 0, s >>>( n, ri, ci, rows, cols, cbits, S.keys, S.idx, S.flag );
       B2S_TRY_CUDA( cudaGetLastError() );
    }
    int bad = 0;
-   B2S_TRY( copy_d2h( &bad, flag.p, sizeof( int ), s ) );
+   B2S_TRY( copy_d2h( &bad, S.flag, sizeof( int ), s ) );
    if( bad ) {
       set_error( "triplet index outside the %d x %d matrix", rows, cols );
       return B2S_INVALID_ARG;
    }
-   if( n > 1 ) {
-      B2S_TRY( keys2.alloc( (size_t) n * sizeof( uint64_t ) ) );
-      B2S_TRY( idx2.alloc( (size_t) n * sizeof( int32_t ) ) );
-      B2S_TRY( radix_sort( keys, idx, keys2, idx2, n, rbits + cbits, s ) );
-      keys2.release();
-      idx2.release();
-   }
+   B2S_TRY( radix_sort( S, n, rbits + cbits, s ) );
    // runs -> unique positions; row capacities (triplet counts)
-   DevBuf head, caps, rcount, off64, off;
-   B2S_TRY( head.alloc( (size_t) std::max< int64_t >( n, 1 ) * sizeof( int64_t ) ) );
-   B2S_TRY( caps.alloc( (size_t) std::max( rows, 1 ) * sizeof( int32_t ) ) );
-   B2S_TRY( rcount.alloc( (size_t) std::max( rows, 1 ) * sizeof( int32_t ) ) );
-   B2S_TRY_CUDA( cudaMemsetAsync( caps.p, 0, (size_t) std::max( rows, 1 ) * sizeof( int32_t ), s ) );
-   B2S_TRY_CUDA( cudaMemsetAsync( rcount.p, 0, (size_t) std::max( rows, 1 ) * sizeof( int32_t ), s ) );
+   int64_t* head = reinterpret_cast< int64_t* >( S.keys2 );
+   const size_t m = (size_t) rows + 1;
+   Pieces C, O;
+   const size_t p_caps = C.add< int32_t >( m ), p_rcount = C.add< int32_t >( m );
+   const size_t p_off64 = O.add< int64_t >( m ), p_off = O.add< int32_t >( m );
+   B2S_TRY( C.buf.alloc( C.used ) );
+   int32_t *caps = C.at< int32_t >( p_caps ), *rcount = C.at< int32_t >( p_rcount );
+   B2S_TRY_CUDA( cudaMemsetAsync( caps, 0, C.used, s ) );
    int64_t nu = 0;
    if( n > 0 ) {
-      coo_heads_kernel<<< grid_of( n ), 256, 0, s >>>( n, keys.as< uint64_t >(), cbits, head.as< int64_t >(),
-                                                       caps.as< int32_t >() );
+      coo_heads_kernel<<< grid_of( n ), 256, 0, s >>>( n, S.keys, cbits, head, caps );
       B2S_TRY_CUDA( cudaGetLastError() );
       int64_t last_head = 0;
-      B2S_TRY( copy_d2h( &last_head, head.as< int64_t >() + n - 1, sizeof( int64_t ), s ) );
-      B2S_TRY( scan_exclusive_i64( head.as< int64_t >(), n, s ) );
-      B2S_TRY( copy_d2h( &nu, head.as< int64_t >() + n - 1, sizeof( int64_t ), s ) );
+      B2S_TRY( copy_d2h( &last_head, head + n - 1, sizeof( int64_t ), s ) );
+      B2S_TRY( scan_exclusive_i64( head, n, s ) );
+      B2S_TRY( copy_d2h( &nu, head + n - 1, sizeof( int64_t ), s ) );
       nu += last_head;
    }
    if( nu > INT32_MAX ) {
@@ -584,31 +630,28 @@ assemble( b2s_format format, b2s_dtype dtype, int32_t rows, int32_t cols, int64_
    B2S_TRY( ucol.alloc( (size_t) std::max< int64_t >( nu, 1 ) * sizeof( int32_t ) ) );
    B2S_TRY( uval.alloc( (size_t) std::max< int64_t >( nu, 1 ) * sizeof( Real ) ) );
    if( n > 0 ) {
-      coo_merge_kernel< Real, Tin ><<< grid_of( n ), 256, 0, s >>>( n, keys.as< uint64_t >(), idx.as< int32_t >(), vals,
-                                                                    head.as< int64_t >(), cbits, add, ucol.as< int32_t >(),
-                                                                    uval.as< Real >(), rcount.as< int32_t >() );
+      coo_merge_kernel< Real, Tin ><<< grid_of( n ), 256, 0, s >>>( n, S.keys, S.idx, vals,
+                                                                    head, cbits, add, ucol.as< int32_t >(),
+                                                                    uval.as< Real >(), rcount );
       B2S_TRY_CUDA( cudaGetLastError() );
    }
-   keys.release();
-   idx.release();
-   head.release();
-   B2S_TRY( off64.alloc( ( (size_t) rows + 1 ) * sizeof( int64_t ) ) );
-   B2S_TRY( off.alloc( ( (size_t) rows + 1 ) * sizeof( int32_t ) ) );
-   counts_to_i64_kernel<<< grid_of( (int64_t) rows + 1 ), 256, 0, s >>>( rcount.as< int32_t >(), rows,
-                                                                          off64.as< int64_t >() );
+   W.buf.release();
+   B2S_TRY( O.buf.alloc( O.used ) );
+   int64_t* off64 = O.at< int64_t >( p_off64 );
+   int32_t* off = O.at< int32_t >( p_off );
+   counts_to_i64_kernel<<< grid_of( (int64_t) m ), 256, 0, s >>>( rcount, rows, off64 );
    B2S_TRY_CUDA( cudaGetLastError() );
-   B2S_TRY( scan_exclusive_i64( off64.as< int64_t >(), (int64_t) rows + 1, s ) );
-   i64_to_i32_kernel<<< grid_of( (int64_t) rows + 1 ), 256, 0, s >>>( off64.as< int64_t >(), (int64_t) rows + 1,
-                                                                      off.as< int32_t >() );
+   B2S_TRY( scan_exclusive_i64( off64, (int64_t) m, s ) );
+   i64_to_i32_kernel<<< grid_of( (int64_t) m ), 256, 0, s >>>( off64, (int64_t) m, off );
    B2S_TRY_CUDA( cudaGetLastError() );
    int64_t caps_total = n;
-   const int32_t* caps_used = caps.as< int32_t >();
+   const int32_t* caps_used = caps;
    if( caps_user ) {
-      B2S_TRY( user_capacities( caps_user, rcount.as< int32_t >(), rows, caps_total, s ) );
+      B2S_TRY( user_capacities( caps_user, rcount, rows, caps_total, s ) );
       caps_used = caps_user;
    }
-   return matrix_from_assembled( format, dtype, rows, cols, nu, off.as< int32_t >(), ucol.as< int32_t >(), uval.p,
-                                 caps_used, caps_total, o, s, out );
+   return matrix_from_assembled( format, dtype, rows, cols, nu, off, ucol.as< int32_t >(), uval.p, caps_used, caps_total,
+                                 o, s, out );
 }
 
 // ---------------------------------------------------------------------------
