@@ -1806,7 +1806,12 @@ build_row_patterns( b2s_matrix_t* A, cudaStream_t s )
    // allocation (another one, freed right away, took longer than the search)
    const size_t lists = ( kMaxPatterns + 1 + kMaxPatternOffsets ) * sizeof( int32_t );
    const size_t at = ( lists + (size_t) ids + 255 ) / 256 * 256;
-   B2S_TRY( A->pat.alloc( at + sizeof( PatternWork ) ) );
+   const b2s_status st = A->pat.alloc( at + sizeof( PatternWork ) );
+   if( st == B2S_OOM ) {  // a matrix that just fits: its products read the columns
+      clear_error();
+      return B2S_OK;
+   }
+   B2S_TRY( st );
    // ids of strip ranks past the rows: pattern 0, never stored
    B2S_TRY_CUDA( cudaMemsetAsync( A->pat.p, 0, A->pat.bytes, s ) );
    PatternWork* W = reinterpret_cast< PatternWork* >( static_cast< char* >( A->pat.p ) + at );
