@@ -117,3 +117,32 @@ def test_small_mixed_requests_run_in_fp64(b2s_lib, cuda):
         assert r["true_residual"] <= 1e-10 and r["refinements"] == 0
         # routed requests are exactly the plain FP64 solves
         assert np.array_equal(xr, xp) and r["iterations"] == pl["iterations"], name
+
+
+def test_admission_counts_incomplete_factors(b2s_lib, cuda):
+    """The estimated bytes cover the factors and the plans of their substitutions, measured
+    as what a solver with ILU(0) holds beyond one without."""
+    from b2s import workloads as W
+    csr = W.convdiff3d(64, seed=1)
+    n = len(csr[0]) - 1
+    A = b2s_lib.SparseMatrix.from_csr(*csr[:3], n)
+    held = {}
+    for precond in ("none", "ilu0"):
+        cuda.cuda.synchronize()
+        before = cuda.cuda.mem_get_info()[0]
+        s = b2s_lib.BICGStab()
+        s.setMatrix(A)
+        s.setPreconditioner(precond)
+        s._ensure()
+        held[precond] = before - cuda.cuda.mem_get_info()[0]
+        del s
+    estimate = {}
+    srv = b2s_lib.Server(max_inflight=1)
+    for precond in ("none", "ilu0"):
+        opts = b2s_lib.solve_opts("bicgstab", tol=1e-8)
+        opts.preconditioner = b2s_lib.PRECONDITIONERS[precond]
+        r = srv.wait(srv.submit(csr, np.ones(n), np.zeros(n), opts), timeout=300)
+        assert r["ok"], r
+        estimate[precond] = r["device_bytes"]
+    srv.close()
+    assert estimate["ilu0"] - estimate["none"] >= held["ilu0"] - held["none"] - (8 << 20)  # 2 MB pages

@@ -64,8 +64,9 @@ struct ServerReq
 };
 
 // Device bytes a request holds at its peak: the matrix (CSR arrays, window
-// tables, diagonal, FP32 copy for mixed precision, build temporaries), the
-// solver's vectors, reduction scratch and, for GMRES, the Krylov basis.
+// tables, diagonal, row patterns, FP32 copy for mixed precision, build
+// temporaries), the solver's vectors, reduction scratch, for GMRES the Krylov
+// basis, and incomplete factors with the plans of their substitutions.
 static int64_t
 estimate_bytes( const b2s_request& r )
 {
@@ -76,6 +77,7 @@ estimate_bytes( const b2s_request& r )
    m += nnz * ( 8 + 4 ) + ( n + 1 ) * 4 + 2 * pad;      // values, columns, offsets
    m += ( nnz / kWinNnzF64 + nnz / kWinNnzF32 + 4 ) * 4;  // window tables
    m += n * 8 + 16 * pad;                                // diagonal, small buffers
+   m += n + 32 * 1024;                                   // row patterns, the table of their search
    if( r.format != B2S_CSR )
       m += nnz * ( 8 + 4 ) + n * 16;                     // padded layout (CSR staging freed later)
    m += ( n + 1 ) * 4 + nnz * ( 4 + 8 ) + n * 4;          // build temporaries
@@ -92,6 +94,12 @@ estimate_bytes( const b2s_request& r )
    if( r.opts.solver == B2S_BICGSTABL ) {
       const int64_t L = std::max( r.opts.bicgstab_ell, 1 );
       s += 2 * ( L + 1 ) * ( ( n + 31 ) / 32 * 32 ) * es + ( L * L + 4 * ( L + 1 ) ) * 8 + 64;
+   }
+   if( r.opts.preconditioner == B2S_PRECOND_ILU0 || r.opts.preconditioner == B2S_PRECOND_ILUT ) {
+      // ILUT adds up to ilut_p entries to each row's part of L and of U
+      const int64_t nf = nnz + ( r.opts.preconditioner == B2S_PRECOND_ILUT ? 2 * (int64_t) r.opts.ilut_p * n : 0 );
+      s += nf * ( 8 + 4 ) + n * ( 4 * 5 + 2 * 8 );        // factors, pattern, positions, flags, orders, scratch
+      s += 2 * n * 50 + 3 * nf * ( 8 + 4 );               // both plans: up to three lanes and slots for each in use
    }
    return m + s + ( 2 << 20 );
 }
