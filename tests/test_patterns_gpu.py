@@ -6,6 +6,8 @@ and after the columns were permuted in place.
 
 Each row within the forward error bound of its dot product,
 2 (L + 3) u (|alpha| (|A| |x|)_i + |beta y0_i|)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -50,6 +52,8 @@ CASES = {
     "five_below": lambda: _stencil(N - 1, [-300, -1, 0, 1, 300]),
     "five": lambda: _stencil(N, [-300, -1, 0, 1, 300]),
     "five_odd": lambda: _stencil(N + 33, [-300, -1, 0, 1, 300], seed=2),
+    # whole slices of ChunkedEllpack: one chunk per row, which its pattern kernel needs
+    "five_chunks": lambda: _stencil(391 * 256, [-300, -1, 0, 1, 300], seed=4),
     "seven_zeros": lambda: _stencil(N + 31, [-2500, -50, -1, 0, 1, 50, 2500], seed=3, zeros=True),
     "wide": lambda: _stencil(N, [0, 3, 90000], cols=N + 70000),
     "tall": lambda: _stencil(N + 1, [-90000, -3, 0], cols=N // 2),
@@ -106,3 +110,22 @@ def test_columns_permuted_in_place(b2s_lib, cuda, oracle, segments):
         M = b2s_lib.SparseMatrix.from_csr(off, col, val, cols, segments=segments)
         M.permuteColumns(iperm)
         _check(b2s_lib, cuda, oracle, M, (off, iperm[col].astype(np.int32), val, cols), "double", segments)
+
+
+def test_layouts_that_keep_patterns(b2s_lib, cuda):
+    """By the memory that a matrix holds before and after its columns are shuffled beyond any
+    pattern: ChunkedEllpack in FP32 reads its columns faster, the others keep patterns."""
+    from b2s._abi import MatrixInfo
+    n = 391 * 256
+    off, col, val, cols = _stencil(n, [-300, -1, 0, 1, 300])
+    shuffle = np.random.default_rng(1).permutation(n).astype(np.int32)
+    for segments, _ in LAYOUTS:
+        for real in ("double", "float"):
+            M = b2s_lib.SparseMatrix.from_csr(off, col, val, cols, segments=segments, real=real)
+            before = M.info.device_bytes
+            M.permuteColumns(shuffle)
+            info = MatrixInfo()
+            assert b2s_lib.lib.b2s_matrix_get_info(M.handle, C.byref(info)) == b2s_lib.OK
+            after = info.device_bytes
+            kept = not (segments == "ChunkedEllpack" and real == "float")
+            assert (before - after >= n) == kept, (segments, real, before - after)

@@ -1801,11 +1801,14 @@ spmv_dispatch( const b2s_matrix_t* A, const Real* values, const Real* x, int32_t
       case B2S_CHUNKED_ELLPACK: {
          const int grid = (int) std::min< int64_t >( std::max( A->numberOfSlices, 1 ),
                                                      std::min< int64_t >( (int64_t) num_sms() * 8, kMaxReduceGrid ) );
-         if( patterns ) {
-            chunked_pattern_kernel< Real, Sink ><<< grid, kChunksInSlice, 0, s >>>(
-               A->patterns(), values, A->cslices.as< ChunkSlice >(), A->rowToSlice.as< int32_t >(), x, rb, re, sink, rs );
+         if constexpr( sizeof( Real ) == 8 ) {  // build_row_patterns: slower in FP32
+            if( patterns ) {
+               chunked_pattern_kernel< Real, Sink ><<< grid, kChunksInSlice, 0, s >>>(
+                  A->patterns(), values, A->cslices.as< ChunkSlice >(), A->rowToSlice.as< int32_t >(), x, rb, re, sink, rs );
+               break;
+            }
          }
-         else if( A->chunk_single ) {
+         if( A->chunk_single ) {
             if( skip )
                chunked1_kernel< Real, true, Sink ><<< grid, kChunksInSlice, 0, s >>>(
                   col, values, A->cslices.as< ChunkSlice >(), A->rowToSlice.as< int32_t >(), x, rb, re, sink, rs );
