@@ -45,9 +45,10 @@ grid_n( int64_t n )
 
 // Blocks of the substitutions, or none when the rows do not suit a lane per
 // row. A step across blocks goes through L2, one inside a block through shared
-// memory, so blocks are large; but a block's warps share one SM. Measured with
-// 2,048 / 8,192 / 16,384 rows at least: 32^3 stencil 155 / 132 / 170 us, 64^3
-// 321 / 284 / 256 us, 2D 140^2 285 / 234 / 228 us.
+// memory, so blocks are large; but a block's warps share one SM. Blocks take at
+// most kTrsvRows rows while there are SMs for more blocks, then equal shares.
+// Measured with 2,048 / 8,192 / 16,384 rows at most: 32^3 stencil 155 / 132 /
+// 170 us, 64^3 321 / 284 / 256 us, 2D 140^2 285 / 234 / 228 us.
 // A lane walks its row alone: rows of up to kTrsvMeanRow factor entries on
 // average, none longer than kTrsvMaxRow.
 constexpr int32_t kTrsvRows = 8192;

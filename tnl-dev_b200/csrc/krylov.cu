@@ -2216,7 +2216,7 @@ true_residual( b2s_solver_t* S, const Real* vals, const Real* b, const Real* x, 
    double* d_out = &S->ctl_buf.as< Ctl >()->outer_norm;  // reuse two doubles of the control block
    TrueResSink< Real > sink{ b, d_out };
    B2S_TRY( ( spmv_dispatch< Real, TrueResSink< Real > >( S->A, vals, x, 0, S->A->rows, sink, S->scr.slot( 9 ), S->cs ) ) );
-   double* h = &S->h_ctl->outer_norm;  // the host mirror is page-locked
+   double* h = &S->h_ctl->outer_norm;  // the host mirror, page-locked outside the server
    B2S_TRY_CUDA( cudaMemcpyAsync( h, d_out, 2 * sizeof( double ), cudaMemcpyDeviceToHost, S->cs ) );
    B2S_TRY_CUDA( cudaStreamSynchronize( S->cs ) );
    res = h[ 1 ] > 0 ? h[ 0 ] / h[ 1 ] : h[ 0 ];

@@ -50,9 +50,9 @@ constexpr int kClusterBlocks = 8;
 // blocks (CG, 1,024 rows: 3.4 us per iteration)
 constexpr int kClusterRows = 16384;
 static_assert( kClusterRows <= 4 * kClusterBlocks * kResBlock, "four rows per thread" );
-// Rows per block below which another block costs more in its meetings than it
-// takes off the others' rows.
-constexpr int kResMinRows = 256;
+// Beyond one cluster, blocks take at most this many rows while there are SMs
+// for more blocks, then equal shares.
+constexpr int kResBlockRows = 256;
 struct MeetSlots
 {
    double v[ 2 ][ 2 ][ kResMaxBlocks ];  // [meeting's parity][value][block]
@@ -506,7 +506,7 @@ resident_shape( const b2s_matrix_t* A, int solver, size_t es )
       if( fits( rows ) )
          return ResidentShape{ blocks, rows, true };
    }
-   const int want = std::max( 1, std::min( num_sms(), ( n + kResMinRows - 1 ) / kResMinRows ) );
+   const int want = std::max( 1, std::min( num_sms(), ( n + kResBlockRows - 1 ) / kResBlockRows ) );
    const int rows = ( n + want - 1 ) / want;
    if( fits( rows ) )
       return ResidentShape{ ( n + rows - 1 ) / rows, rows, false };
@@ -576,9 +576,8 @@ launch_resident_rows( const ResidentArgs< Real >& a, int blocks, cudaStream_t s 
       return launch_resident< Real, 2, BICG, CLUSTER >( a, blocks, s );
    if( rpt <= 4 )
       return launch_resident< Real, 4, BICG, CLUSTER >( a, blocks, s );
-   if constexpr( ! CLUSTER ) {
+   if constexpr( ! CLUSTER && ! ( BICG && sizeof( Real ) == 8 ) )  // as many as resident_shape gives
       return launch_resident< Real, 8, BICG, CLUSTER >( a, blocks, s );
-   }
    set_error( "resident solver: %d rows per block", a.rows_per_block );
    return B2S_UNSUPPORTED;
 }

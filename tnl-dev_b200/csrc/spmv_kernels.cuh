@@ -580,10 +580,10 @@ load_patterns( const RowPatterns& P, PatternSmem& S )
       S.off[ i ] = __ldg( P.off + i );
 }
 
-// CSR row groups with patterns: csr_group_kernel without the columns. The
-// row-group kernels issue instructions most of the time (0.6-0.7 per cycle and
-// scheduler), so this one counts them: 32-bit row arithmetic, eight elements at
-// a time under predicates.
+// CSR row groups with patterns: csr_group_kernel without the columns. In FP32
+// it issues instructions most of the time (0.68 per cycle and scheduler on the
+// 128^3 Laplacian, 0.46 in FP64), so it counts them: 32-bit row arithmetic,
+// eight elements at a time under predicates.
 // kCsrPatStages groups of values are in flight or being summed per warp, and a
 // warp takes groups of 64 rows, lane l rows l and l + 32, which share the
 // group's staging. 128^3 / 160^3 Laplacian, us:
@@ -736,14 +736,6 @@ ld_values( const double* p, double ( &v )[ 2 ] )
    v[ 0 ] = q.x;
    v[ 1 ] = q.y;
 }
-__device__ __forceinline__ void
-ld_values( const double* p, double ( &v )[ 4 ] )
-{
-   asm( "ld.global.nc.L1::no_allocate.v4.f64 {%0,%1,%2,%3}, [%4];"
-        : "=d"( v[ 0 ] ), "=d"( v[ 1 ] ), "=d"( v[ 2 ] ), "=d"( v[ 3 ] )
-        : "l"( p ) );
-}
-
 // slots whose loads are in flight together, per row of a thread (eight took
 // the registers of three resident blocks: 37 against 31 us on the 128^3
 // Laplacian in FP64)
