@@ -139,3 +139,28 @@ def test_resident_single_and_mixed_precision(b2s_lib, cuda, oracle, kind, n):
     assert s.solve(cuda.tensor(b, dtype=cuda.float32, device="cuda"), x)
     r = np.linalg.norm(oracle.spmv("csr", "col", csr, x.cpu().numpy().astype(np.float64)) - b)
     assert r <= 1e-3 * np.linalg.norm(b)  # the recurrence's residue, and FP32's rounding on top
+
+
+# beyond one cluster a block takes n / 148 rows, here 541 to 2,095 (the last block fewer):
+# two, four and eight to a thread; FP64 BiCGStab at most four
+@pytest.mark.parametrize("n", [80_001, 160_003, 310_005])
+@pytest.mark.parametrize("kind", ["cg", "bicgstab"])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_resident_rows_per_thread(b2s_lib, cuda, oracle, n, kind, mixed):
+    csr = _spd(n, [1, 700])
+    b = np.random.default_rng(8).uniform(-1, 1, n)
+    for precond in (None, "diagonal"):
+        want = oracle.solve(kind, csr, b, rtol=1e-10, precond=precond is not None)
+        d = csr[2][csr[1] == np.repeat(np.arange(n), np.diff(csr[0]))]  # the bound: test_resident_vs_oracle
+        bound = 4e-10 * (np.linalg.norm(b) if precond is None else np.max(d) * np.linalg.norm(b / d))
+        for segments in ("CSR", "SlicedEllpack", "Ellpack"):
+            M = b2s_lib.SparseMatrix.from_csr(*csr[:3], n, segments=segments, keep_fp32_copy=mixed)
+            s = _solver(b2s_lib, kind)
+            s.setMatrix(M)
+            s.setPreconditioner(precond)
+            s.setConvergenceResidue(1e-10)
+            s.setPrecision(mixed)
+            x = cuda.zeros(n, dtype=cuda.float64, device="cuda")
+            assert s.solve(cuda.tensor(b, device="cuda"), x), (precond, segments)
+            err = np.max(np.abs(x.cpu().numpy() - want["x"]))
+            assert err <= bound, (precond, segments, err, bound)
