@@ -110,13 +110,15 @@ struct ResidentArgs
 
 // All blocks' sums of NV values, the same in every thread of every block;
 // everything a block wrote before is visible to all after. false: gave up.
-// `meeting` counts the launch's meetings, `base` is the slots' count before it.
+// `meeting` counts the launch's meetings; *due, thread 0's, is the slots' count
+// after the last one (in shared memory: as 64 bits in registers it cost BiCGStab
+// 2 %).
 // `fin( totals )` runs in one thread of every block before the others go on:
 // the scalar work, which every block does alike (a double division or root in
 // all 16 warps takes longer than in one).
 template< int NV, bool CLUSTER, class Fin >
 __device__ __forceinline__ bool
-meet( double ( &v )[ NV ], MeetSlots* S, int looks, unsigned& meeting, unsigned long long base, Fin&& fin )
+meet( double ( &v )[ NV ], MeetSlots* S, int looks, unsigned& meeting, unsigned long long* due, Fin&& fin )
 {
    __shared__ double sh[ NV ][ kResBlock / 32 ];
    __shared__ double part[ 2 ][ NV ];
@@ -157,7 +159,7 @@ meet( double ( &v )[ NV ], MeetSlots* S, int looks, unsigned& meeting, unsigned 
             S->v[ set ][ k ][ blockIdx.x ] = v[ k ];
          meet_fence();
          atomicAdd( &S->count, 1ull );
-         const unsigned long long want = base + (unsigned long long) meeting * (unsigned) G;
+         const unsigned long long want = *due += (unsigned) G;
          unsigned long long c;
          for( int it = 0; ( c = *(volatile unsigned long long*) &S->count ) < want; it++ )
             if( it >= looks && atomicCAS( &S->count, c, c | kMeetOff ) == c ) {
@@ -269,11 +271,13 @@ resident_kernel( ResidentArgs< Real > a )
          a.ctl->gave_up = 1;
    };
    unsigned meeting = 0;
-   const unsigned long long base = *(volatile unsigned long long*) &a.slots->base;
+   __shared__ unsigned long long due;  // thread 0's: the count that the last meeting waited for
+   if( tid == 0 )
+      due = *(volatile unsigned long long*) &a.slots->base;
    // every block's start (its copy of ctl included) precedes any end
    {
       double one[ 1 ] = { 0.0 };
-      if( ! meet< 1, CLUSTER >( one, a.slots, a.looks, meeting, base, []( const double* ) {} ) )
+      if( ! meet< 1, CLUSTER >( one, a.slots, a.looks, meeting, &due, []( const double* ) {} ) )
          return give_up();
    }
    Real *pa = a.v.p, *pb = a.v.p2;      // p of the last direction, and the one being formed
@@ -301,7 +305,7 @@ resident_kernel( ResidentArgs< Real > a )
             Ap[ j ] = s;
             acc[ 0 ] += (double) s * (double) p[ j ];
          }
-         if( ! meet< 1, CLUSTER >( acc, a.slots, a.looks, meeting, base, [ & ]( const double* t ) {
+         if( ! meet< 1, CLUSTER >( acc, a.slots, a.looks, meeting, &due, [ & ]( const double* t ) {
                 // CgApSink::finish
                 c.s2 = t[ 0 ];
                 if( c.s2 == 0.0 ) {
@@ -340,7 +344,7 @@ resident_kernel( ResidentArgs< Real > a )
             }
             acc[ 0 ] += (double) r[ j ] * (double) zz[ j ];
          }
-         if( ! meet< 1, CLUSTER >( acc, a.slots, a.looks, meeting, base, [ & ]( const double* t ) { CgUpdateFin{}( c, t ); } ) )
+         if( ! meet< 1, CLUSTER >( acc, a.slots, a.looks, meeting, &due, [ & ]( const double* t ) { CgUpdateFin{}( c, t ); } ) )
             return give_up();
          live = ! c.done;
          if( live ) {
@@ -374,7 +378,7 @@ resident_kernel( ResidentArgs< Real > a )
             acc[ 0 ] += (double) s * (double) __ldg( a.v.r_ast + i );
          }
          double a1[ 1 ] = { acc[ 0 ] };
-         if( ! meet< 1, CLUSTER >( a1, a.slots, a.looks, meeting, base,
+         if( ! meet< 1, CLUSTER >( a1, a.slots, a.looks, meeting, &due,
                                    [ & ]( const double* t ) { c.bi_alpha = c.rho / t[ 0 ]; } ) )
             return give_up();
          if( ! first ) {
@@ -407,7 +411,7 @@ resident_kernel( ResidentArgs< Real > a )
             acc[ 0 ] += (double) s * (double) s_[ j ];
             acc[ 1 ] += (double) s * (double) s;
          }
-         if( ! meet< 2, CLUSTER >( acc, a.slots, a.looks, meeting, base,
+         if( ! meet< 2, CLUSTER >( acc, a.slots, a.looks, meeting, &due,
                                    [ & ]( const double* t ) { c.omega = t[ 0 ] / t[ 1 ]; } ) )
             return give_up();
          const Real omega = (Real) c.omega;
@@ -423,7 +427,7 @@ resident_kernel( ResidentArgs< Real > a )
             acc[ 0 ] += (double) r[ j ] * (double) __ldg( a.v.r_ast + i );
             acc[ 1 ] += (double) r[ j ] * (double) r[ j ];
          }
-         if( ! meet< 2, CLUSTER >( acc, a.slots, a.looks, meeting, base, [ & ]( const double* t ) { BiXrFin{ a.eps2, 0 }( c, t ); } ) )
+         if( ! meet< 2, CLUSTER >( acc, a.slots, a.looks, meeting, &due, [ & ]( const double* t ) { BiXrFin{ a.eps2, 0 }( c, t ); } ) )
             return give_up();
          if( c.restart_flag )
             break;
@@ -439,7 +443,7 @@ resident_kernel( ResidentArgs< Real > a )
    // every block has left the gathers of its last direction: the vectors may be put back
    {
       double one[ 1 ] = { 0.0 };
-      if( ! meet< 1, CLUSTER >( one, a.slots, a.looks, meeting, base, []( const double* ) {} ) )
+      if( ! meet< 1, CLUSTER >( one, a.slots, a.looks, meeting, &due, []( const double* ) {} ) )
          return give_up();
    }
 #pragma unroll
@@ -473,7 +477,7 @@ resident_kernel( ResidentArgs< Real > a )
          o.alpha = c.alpha;
          o.beta = c.beta;
       }
-      a.slots->base = base + (unsigned long long) meeting * gridDim.x;
+      a.slots->base = due;
    }
    if constexpr( CLUSTER )
       cooperative_groups::this_cluster().sync();  // the others may still read this block's sums
