@@ -15,6 +15,18 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200) and the built libb2sparse.so")
 
 
+@pytest.hookimpl(hookwrapper=True)
+def pytest_runtest_makereport(item, call):
+    """Tests against TNL's own host build are skipped where oracle/_ref is not
+    built (it needs TNL's headers); every other failure stays one."""
+    outcome = yield
+    report = outcome.get_result()
+    if call.excinfo is not None and call.excinfo.errisinstance(FileNotFoundError):
+        if "libtnlref.so is not built" in str(call.excinfo.value):
+            report.outcome = "skipped"
+            report.longrepr = (str(item.path), item.location[1], "Skipped: oracle/_ref is not built on this machine")
+
+
 @pytest.fixture(scope="session")
 def oracle():
     from oracle import Oracle
